@@ -546,22 +546,20 @@ __device__ __forceinline__ int table_slot(int *keys, int *vals, long long tsz, i
     }
 }
 
-// Warp-cooperative Galerkin product with the same discovery and accumulation
-// order as the sequential traversal (R row I -> A row i -> P row j): the 32
-// lanes take 32 consecutive products of the traversal; lanes with the same
-// coarse column are grouped (__match_any_sync) and the group's lowest lane adds
-// the members' products to the column's sum one by one in lane order, so
-// every column's sum is formed in traversal order.  New columns get slots in
-// order of first occurrence.  The row's column table lives in shared memory,
-// in two sizes: every row is first tried with a 256-entry table (8 warps per
-// block, many blocks per SM: the rows of the fine levels are short), a row
-// with more than 128 columns again with a 2,048-entry table (2 warps per
-// block), and a row with more than 1,024 columns is redone by
-// rap_fallback_kernel (one thread, table in global memory).  The table only
-// indexes the columns: a row's result does not depend on which size held it.
-// overflow[I]: 0 small table, 1 large table, 2 fallback.
-static constexpr int kRapTableS = 256, kRapWarpsS = 8;   // small tier: entries per warp, warps per block
-static constexpr int kRapTableL = 2048, kRapWarpsL = 2;  // large tier
+// Galerkin product with the same discovery and accumulation order as the
+// sequential traversal (R row I -> A row i -> P row j).  32 lanes take 32
+// consecutive products of the traversal; lanes with the same coarse column are
+// grouped (__match_any_sync) and the group's lowest lane adds the members'
+// products to the column's sum one by one in lane order, so every column's sum
+// is formed in traversal order.  New columns get slots in order of first
+// occurrence.  The row's column table lives in shared memory and only indexes
+// the columns: a row's result does not depend on which kernel formed it.
+// tier[I]: 0 rap_warp_kernel, a warp per row with a 256-entry table (rows of
+// fewer than kRapPairs pairs (A entry, its R entry) and at most 128 columns);
+// 1 rap_block_kernel, a block per row; 2 rap_fallback_kernel (one thread, table
+// in global memory: rows whose columns overflow the block's tables).
+static constexpr int kRapTable = 256, kRapWarps = 8;  // warp kernel: entries per warp, warps per block
+static constexpr int kRapPairs = 192;
 
 template <int TBL>
 __device__ __forceinline__ int rap_find(const int *keys, int J) {
@@ -584,15 +582,15 @@ __device__ __forceinline__ int rap_insert(int *keys, int J) {
     }
 }
 
-template <bool FILL, int TBL, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS)
+template <bool FILL>
+__global__ void __launch_bounds__(32 * kRapWarps)
     rap_warp_kernel(int nrows, const int *__restrict__ ria, const int *__restrict__ rja,
                     const double *__restrict__ ra, const int *__restrict__ aia, const int *__restrict__ aja,
                     const double *__restrict__ aa, const int *__restrict__ pia, const int *__restrict__ pja,
-                    const double *__restrict__ pa, int *__restrict__ cnt, unsigned char *__restrict__ overflow,
+                    const double *__restrict__ pa, int *__restrict__ cnt, unsigned char *__restrict__ tier,
                     const int *__restrict__ cia, int *__restrict__ cja, double *__restrict__ ca) {
+    constexpr int TBL = kRapTable, WARPS = kRapWarps;
     constexpr int kMaxCols = TBL / 2;  // columns a warp row may hold
-    constexpr unsigned char kTier = TBL == kRapTableS ? 0 : 1;
     extern __shared__ __align__(16) unsigned char rap_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *keys = reinterpret_cast<int *>(rap_smem) + warp * TBL;
@@ -600,8 +598,7 @@ __global__ void __launch_bounds__(32 * WARPS)
     double *vals = reinterpret_cast<double *>(rap_smem + (size_t)2 * WARPS * TBL * sizeof(int)) + warp * TBL;
     const unsigned FULL = 0xffffffffu;
     for (int I = blockIdx.x * WARPS + warp; I < nrows; I += gridDim.x * WARPS) {
-        // the small tier counts every row; every other pass takes the rows of its own tier
-        if ((FILL || kTier == 1) && overflow[I] != kTier) continue;
+        if (tier[I] != 0) continue;
         for (int t = lane; t < TBL; t += 32) keys[t] = -1;
         __syncwarp();
         int next = 1;
@@ -699,7 +696,7 @@ __global__ void __launch_bounds__(32 * WARPS)
             }
         }
         if (over) {
-            if (!FILL && lane == 0) overflow[I] = kTier + 1;  // to the next tier
+            if (!FILL && lane == 0) tier[I] = 1;
             __syncwarp();
             continue;
         }
@@ -719,7 +716,274 @@ __global__ void __launch_bounds__(32 * WARPS)
     }
 }
 
-// Thread-per-row fallback for the rows the warp kernel could not hold.
+// tier[I] = 1 for the rows with at least kRapPairs pairs, else 0
+__global__ void rap_tier_kernel(int nrows, const int *__restrict__ ria, const int *__restrict__ rja,
+                                const int *__restrict__ aia, unsigned char *__restrict__ tier) {
+    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+    if (I >= nrows) return;
+    int pairs = 0;
+    for (int r = ria[I]; r < ria[I + 1] && pairs < kRapPairs; ++r) {
+        const int i = rja[r];
+        pairs += aia[i + 1] - aia[i];
+    }
+    tier[I] = pairs >= kRapPairs ? 1 : 0;
+}
+
+// list[0 .. *count) = the rows of tier `which` (in any order)
+__global__ void rap_list_kernel(int nrows, const unsigned char *__restrict__ tier, int which, int *__restrict__ count,
+                                int *__restrict__ list) {
+    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+    if (I < nrows && tier[I] == which) list[atomicAdd(count, 1)] = I;
+}
+
+// One coarse row per block.  The traversal is cut into runs of pairs and these into runs of products;
+// each run is expanded by the whole block (every load of a run is in flight at once: row by row in one
+// warp, the chain of five dependent loads per 32 products was most of the time), then added up from
+// shared memory by eight warps, each for the columns of its own hash class, in traversal order.  A
+// column's first product gives its place: the columns are ranked by it at the end.
+// Newton step's hierarchy of a 63,504-cell system: 10.4 -> 2.5 ms of RAP (the last two products, 1,365
+// and 236 rows of 1,200 to 3,700 pairs, took 9.4 of them).
+static constexpr int kRapParts = 8, kRapPartTable = 256, kRapPartCols = 192;
+static constexpr int kRapRun = 1024;  // products per run
+struct RapBlockSmem {
+    double vals[kRapParts][kRapPartTable];
+    int keys[kRapParts][kRapPartTable];
+    int first[kRapParts][kRapPartTable];
+    double rv[256], pv[256];       // R values; r a of each pair
+    int rpre[257], ra0[256];       // pairs before each R entry; start of its A row
+    int ppre[257], p0[256];        // products before each pair; start of its P row
+    union {
+        struct {
+            double prod[kRapRun];
+            int col[kRapRun];
+        } run;
+        struct {
+            int first[kRapParts * kRapPartCols];
+            unsigned short at[kRapParts * kRapPartCols];
+        } rank;
+    };
+    unsigned short queue[kRapParts][64];
+    int scan[8];
+    int over, ncols;
+    long long base;
+};
+
+// exclusive prefix over the block's 256 threads; *total = the sum (in every thread)
+__device__ __forceinline__ int rap_block_scan(int v, int *scan, int *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    __syncthreads();  // the previous scan's readers are done
+    if (lane == 31) scan[warp] = incl;
+    __syncthreads();
+    int off = 0, sum = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        if (q < warp) off += scan[q];
+        sum += scan[q];
+    }
+    *total = sum;
+    return off + incl - v;
+}
+
+// the last index in [0, n) whose prefix is <= x (pre[0] = 0 <= x)
+__device__ __forceinline__ int rap_owner(const int *pre, int n, int x) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (pre[mid] <= x) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+__global__ void __launch_bounds__(256, 3)
+    rap_block_kernel(const int *__restrict__ list, const int *__restrict__ ria, const int *__restrict__ rja,
+                     const double *__restrict__ ra, const int *__restrict__ aia, const int *__restrict__ aja,
+                     const double *__restrict__ aa, const int *__restrict__ pia, const int *__restrict__ pja,
+                     const double *__restrict__ pa, int *__restrict__ cnt, unsigned char *__restrict__ tier,
+                     unsigned long long *__restrict__ used, long long cap, long long *__restrict__ start,
+                     int *__restrict__ tcol, double *__restrict__ tval) {
+    extern __shared__ __align__(16) unsigned char rap_smem[];
+    RapBlockSmem &S = *reinterpret_cast<RapBlockSmem *>(rap_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned FULL = 0xffffffffu;
+    const int I = list[blockIdx.x];
+    int *keys = S.keys[warp];
+    for (int t = tid; t < kRapParts * kRapPartTable; t += 256) (&S.keys[0][0])[t] = -1;
+    if (tid == 0) {
+        S.over = 0;
+        S.ncols = 0;
+    }
+    __syncthreads();
+    int next = 0;  // columns of this warp's class
+    if ((int)(hash_col(I) >> 29) == warp) {
+        next = 1;
+        if (lane == 0) {  // diagonal first, starting from zero
+            const int h = rap_insert<kRapPartTable>(keys, I);
+            S.first[warp][h] = -1;
+            S.vals[warp][h] = 0.0;
+        }
+    }
+    __syncwarp();
+    bool over = false;
+    int done = 0;  // products of earlier runs
+    // adds queue entries 0..n-1 (n <= 32): products of this warp's class in traversal order
+    auto add = [&](int n) {
+        const bool valid = lane < n;
+        const int t = valid ? S.queue[warp][lane] : 0;
+        const int J = valid ? S.run.col[t] : -1 - lane;  // unique dummy key for idle lanes
+        const double prod = valid ? S.run.prod[t] : 0.0;
+        const unsigned grp = __match_any_sync(FULL, J);
+        const bool leader = valid && lane == __ffs(grp) - 1;
+        int h = leader ? rap_find<kRapPartTable>(keys, J) : -1;
+        const bool fresh = leader && h < 0;
+        const unsigned fresh_mask = __ballot_sync(FULL, fresh);
+        if (next + __popc(fresh_mask) > kRapPartCols) {
+            over = true;  // warp-uniform
+            return;
+        }
+        next += __popc(fresh_mask);
+        if (fresh) {
+            h = rap_insert<kRapPartTable>(keys, J);
+            S.first[warp][h] = done + t;
+        }
+        double acc = leader && !fresh ? S.vals[warp][h] : 0.0;
+        bool starts = fresh;
+        unsigned rem = leader ? grp : 0u;
+        const unsigned steps = __reduce_max_sync(FULL, (unsigned)__popc(rem));
+        for (unsigned it = 0; it < steps; ++it) {
+            const int src = rem ? __ffs(rem) - 1 : lane;
+            const double v = __shfl_sync(FULL, prod, src);
+            if (rem) {
+                acc = starts ? v : acc + v;
+                starts = false;
+                rem &= rem - 1u;
+            }
+        }
+        if (leader) S.vals[warp][h] = acc;
+        __syncwarp();
+    };
+    const int rb = ria[I], re = ria[I + 1];
+    for (int r0 = rb; r0 < re && !S.over; r0 += 256) {
+        const int m = min(256, re - r0);
+        int len = 0, total;
+        if (tid < m) {
+            const int i = rja[r0 + tid];
+            const int k0 = aia[i];
+            len = aia[i + 1] - k0;
+            S.ra0[tid] = k0;
+            S.rv[tid] = ra[r0 + tid];
+        }
+        const int pre = rap_block_scan(len, S.scan, &total);
+        S.rpre[tid] = pre;
+        __syncthreads();
+        for (int pb = 0; pb < total && !S.over; pb += 256) {
+            const int np = min(256, total - pb);
+            int plen = 0, prods;
+            if (tid < np) {
+                const int r = rap_owner(S.rpre, m, pb + tid);
+                const int k = S.ra0[r] + (pb + tid - S.rpre[r]);
+                const int j = aja[k];
+                const int q0 = pia[j];
+                plen = pia[j + 1] - q0;
+                S.p0[tid] = q0;
+                S.pv[tid] = S.rv[r] * aa[k];
+            }
+            const int ppre = rap_block_scan(plen, S.scan, &prods);
+            S.ppre[tid] = ppre;
+            __syncthreads();
+            for (int qb = 0; qb < prods; qb += kRapRun) {
+                const int nq = min(kRapRun, prods - qb);
+#pragma unroll
+                for (int u = 0; u < kRapRun / 256; ++u) {
+                    const int t = tid + 256 * u;
+                    if (t < nq) {
+                        const int o = rap_owner(S.ppre, np, qb + t);
+                        const int q = S.p0[o] + (qb + t - S.ppre[o]);
+                        S.run.col[t] = pja[q];
+                        S.run.prod[t] = S.pv[o] * pa[q];
+                    }
+                }
+                __syncthreads();
+                int qn = 0;
+                for (int t0 = 0; t0 < nq && !over; t0 += 32) {
+                    const int t = t0 + lane;
+                    const bool mine = t < nq && (int)(hash_col(S.run.col[t]) >> 29) == warp;
+                    const unsigned mask = __ballot_sync(FULL, mine);
+                    if (mine) S.queue[warp][qn + __popc(mask & ((1u << lane) - 1u))] = (unsigned short)t;
+                    qn += __popc(mask);
+                    __syncwarp();
+                    if (qn >= 32) {
+                        add(32);
+                        qn -= 32;
+                        const unsigned short v = lane < qn ? S.queue[warp][32 + lane] : 0;
+                        __syncwarp();
+                        if (lane < qn) S.queue[warp][lane] = v;
+                        __syncwarp();
+                    }
+                }
+                if (qn > 0 && !over) add(qn);
+                if (over && lane == 0) S.over = 1;
+                done += nq;
+                __syncthreads();
+                if (S.over) break;
+            }
+        }
+    }
+    __syncthreads();
+    if (S.over) {
+        if (tid == 0) tier[I] = 2;
+        return;
+    }
+    // the columns ranked by their first product
+    for (int t = tid; t < kRapParts * kRapPartTable; t += 256)
+        if ((&S.keys[0][0])[t] >= 0) {
+            const int c = atomicAdd(&S.ncols, 1);
+            S.rank.first[c] = (&S.first[0][0])[t];
+            S.rank.at[c] = (unsigned short)t;
+        }
+    __syncthreads();
+    const int n = S.ncols;
+    if (tid == 0) {
+        S.base = (long long)atomicAdd(used, (unsigned long long)n);
+        cnt[I] = n;
+        start[I] = S.base;
+    }
+    __syncthreads();
+    if (S.base + n > cap) return;  // the caller repeats the pass with room for *used entries
+    for (int c = tid; c < n; c += 256) {
+        const int f = S.rank.first[c];
+        int place = 0;
+        for (int e = 0; e < n; ++e) place += S.rank.first[e] < f;
+        const int t = S.rank.at[c];
+        tcol[S.base + place] = (&S.keys[0][0])[t];
+        tval[S.base + place] = (&S.vals[0][0])[t];
+    }
+}
+
+// the block kernel's rows into A_c, a warp per row
+__global__ void rap_copy_kernel(int nlist, const int *__restrict__ list, const unsigned char *__restrict__ tier,
+                                const long long *__restrict__ start, const int *__restrict__ tcol,
+                                const double *__restrict__ tval, const int *__restrict__ cia, int *__restrict__ cja,
+                                double *__restrict__ ca) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= nlist) return;
+    const int I = list[w];
+    if (tier[I] != 1) return;
+    const int b = cia[I], n = cia[I + 1] - b;
+    const long long t = start[I];
+    for (int e = lane; e < n; e += 32) {
+        cja[b + e] = tcol[t + e];
+        ca[b + e] = tval[t + e];
+    }
+}
+
+// Thread-per-row fallback for the rows the block kernel could not hold.
 template <bool FILL>
 __global__ void rap_fallback_kernel(int nlist, const int *__restrict__ list, const int *__restrict__ ria,
                                     const int *__restrict__ rja, const double *__restrict__ ra,
@@ -771,47 +1035,56 @@ void amg_rap(const CsrView<double> &A, const DeviceCsr &P, const DeviceCsr &R, D
              long long table_budget_entries) {
     (void)table_budget_entries;
     const int nc = P.ncols;
-    const size_t smemS = (size_t)kRapWarpsS * kRapTableS * (2 * sizeof(int) + sizeof(double));
-    const size_t smemL = (size_t)kRapWarpsL * kRapTableL * (2 * sizeof(int) + sizeof(double));
-    static bool attr[64] = {};
-    int dev = 0;
-    JX_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !attr[dev]) {
-        JX_CUDA(cudaFuncSetAttribute(rap_warp_kernel<false, kRapTableL, kRapWarpsL>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemL));
-        JX_CUDA(cudaFuncSetAttribute(rap_warp_kernel<true, kRapTableL, kRapWarpsL>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemL));
-        if (dev >= 0 && dev < 64) attr[dev] = true;
-    }
+    const size_t smemW = (size_t)kRapWarps * kRapTable * (2 * sizeof(int) + sizeof(double));
+    JX_CUDA(cudaFuncSetAttribute(rap_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(RapBlockSmem)));
     DevBuf<int> cnt(nc + 1);
-    DevBuf<unsigned char> over(nc + 1);
+    DevBuf<unsigned char> tier(nc + 1);
     cnt.zero(s);
-    over.zero(s);
-    const int gridS = std::max(1, std::min(div_up(nc, kRapWarpsS), 64 * sm_count()));
-    const int gridL = std::max(1, std::min(div_up(nc, kRapWarpsL), 64 * sm_count()));
+    const int gridW = std::max(1, std::min(div_up(nc, kRapWarps), 64 * sm_count()));
+    // lists of the rows of tiers 1 and 2, their lengths in count[0], count[1]
+    DevBuf<int> d_block(nc > 0 ? nc : 1), d_list(nc > 0 ? nc : 1), count(2);
+    DevBuf<long long> start(nc > 0 ? nc : 1);
+    DevBuf<unsigned long long> used(1);
+    DevBuf<int> tcol;
+    DevBuf<double> tval;
+    count.zero(s);
+    int nblk = 0, nl = 0;
     if (nc > 0) {
-        rap_warp_kernel<false, kRapTableS, kRapWarpsS><<<gridS, 32 * kRapWarpsS, smemS, s>>>(
-            nc, R.ia.get(), R.ja.get(), R.a.get(), A.ia, A.ja, A.a, P.ia.get(), P.ja.get(), P.a.get(), cnt.get(),
-            over.get(), nullptr, nullptr, nullptr);
+        rap_tier_kernel<<<div_up(nc, 128), 128, 0, s>>>(nc, R.ia.get(), R.ja.get(), A.ia, tier.get());
         JX_LAUNCH_CHECK();
-        rap_warp_kernel<false, kRapTableL, kRapWarpsL><<<gridL, 32 * kRapWarpsL, smemL, s>>>(
+        rap_warp_kernel<false><<<gridW, 32 * kRapWarps, smemW, s>>>(
             nc, R.ia.get(), R.ja.get(), R.a.get(), A.ia, A.ja, A.a, P.ia.get(), P.ja.get(), P.a.get(), cnt.get(),
-            over.get(), nullptr, nullptr, nullptr);
+            tier.get(), nullptr, nullptr, nullptr);
         JX_LAUNCH_CHECK();
+        rap_list_kernel<<<div_up(nc, 256), 256, 0, s>>>(nc, tier.get(), 1, count.get(), d_block.get());
+        JX_LAUNCH_CHECK();
+        count.download(&nblk, 1, s);
+        JX_CUDA(cudaStreamSynchronize(s));
     }
-    // rows that overflowed the shared table: thread-per-row with a global table
-    std::vector<unsigned char> h_over(nc > 0 ? nc : 1);
-    over.download(h_over.data(), nc, s);
-    JX_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> list;
-    for (int I = 0; I < nc; ++I)
-        if (h_over[I] == 2) list.push_back(I);
-    const int nl = (int)list.size();
-    DevBuf<int> d_list(nl > 0 ? nl : 1);
+    if (nblk > 0) {
+        // room for 192 columns per row at first; the pass is repeated where the rows have more
+        unsigned long long need = 0;
+        for (long long cap = (long long)nblk * std::min(192, nc);; cap = (long long)need) {
+            tcol.alloc((size_t)cap);
+            tval.alloc((size_t)cap);
+            used.zero(s);
+            rap_block_kernel<<<nblk, 256, sizeof(RapBlockSmem), s>>>(
+                d_block.get(), R.ia.get(), R.ja.get(), R.a.get(), A.ia, A.ja, A.a, P.ia.get(), P.ja.get(), P.a.get(),
+                cnt.get(), tier.get(), used.get(), cap, start.get(), tcol.get(), tval.get());
+            JX_LAUNCH_CHECK();
+            used.download(&need, 1, s);
+            JX_CUDA(cudaStreamSynchronize(s));
+            if (need <= (unsigned long long)cap) break;
+        }
+        rap_list_kernel<<<div_up(nc, 256), 256, 0, s>>>(nc, tier.get(), 2, count.get() + 1, d_list.get());
+        JX_LAUNCH_CHECK();
+        JX_CUDA(cudaMemcpyAsync(&nl, count.get() + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+        JX_CUDA(cudaStreamSynchronize(s));
+    }
     DevBuf<long long> toff(nl + 1);
     DevBuf<int> tkeys, tvals;
     if (nl > 0) {
-        d_list.upload(list.data(), nl, s);
         // table per listed row: 2 x (columns reachable) <= 2 x nc, power of two
         long long t = 16;
         while (t < 2LL * nc) t <<= 1;
@@ -837,13 +1110,15 @@ void amg_rap(const CsrView<double> &A, const DeviceCsr &P, const DeviceCsr &R, D
     Ac.ja.alloc(nnz > 0 ? nnz : 1);
     Ac.a.alloc(nnz > 0 ? nnz : 1);
     if (nc > 0) {
-        rap_warp_kernel<true, kRapTableS, kRapWarpsS><<<gridS, 32 * kRapWarpsS, smemS, s>>>(
+        rap_warp_kernel<true><<<gridW, 32 * kRapWarps, smemW, s>>>(
             nc, R.ia.get(), R.ja.get(), R.a.get(), A.ia, A.ja, A.a, P.ia.get(), P.ja.get(), P.a.get(), nullptr,
-            over.get(), Ac.ia.get(), Ac.ja.get(), Ac.a.get());
+            tier.get(), Ac.ia.get(), Ac.ja.get(), Ac.a.get());
         JX_LAUNCH_CHECK();
-        rap_warp_kernel<true, kRapTableL, kRapWarpsL><<<gridL, 32 * kRapWarpsL, smemL, s>>>(
-            nc, R.ia.get(), R.ja.get(), R.a.get(), A.ia, A.ja, A.a, P.ia.get(), P.ja.get(), P.a.get(), nullptr,
-            over.get(), Ac.ia.get(), Ac.ja.get(), Ac.a.get());
+    }
+    if (nblk > 0) {
+        rap_copy_kernel<<<div_up((long long)nblk * 32, 256), 256, 0, s>>>(
+            nblk, d_block.get(), tier.get(), start.get(), tcol.get(), tval.get(), Ac.ia.get(), Ac.ja.get(),
+            Ac.a.get());
         JX_LAUNCH_CHECK();
     }
     if (nl > 0) {
