@@ -35,20 +35,33 @@
 namespace jxcpr {
 
 namespace {
+// A point of the first pass: its links in its measure's bucket, its measure and state in one 16-byte
+// record, since the greedy touches points in no order a cache could follow (separate arrays: four lines per
+// point instead of one).  Buckets hold measures up to twice the largest initial one: a point's measure grows
+// once per row that depends on it.
+struct Point {
+    int next, prev, measure, cf;
+};
 struct Buckets {
-    std::vector<int> next, prev, head, tail;
+    std::vector<Point> p;
+    std::vector<int> head, tail;
     int maxm = 0;
-    Buckets(int n, int cap) : next(n, -1), prev(n, -1), head(cap, -1), tail(cap, -1) {}
+    explicit Buckets(int n) : p(n) {}
+    void init(int maxmeasure) {
+        head.assign(2 * (size_t)maxmeasure + 2, -1);
+        tail.assign(2 * (size_t)maxmeasure + 2, -1);
+    }
     void enter(int m, int i) {
-        next[i] = -1;
-        prev[i] = tail[m];
-        if (tail[m] >= 0) next[tail[m]] = i; else head[m] = i;
+        p[i].next = -1;
+        p[i].prev = tail[m];
+        if (tail[m] >= 0) p[tail[m]].next = i; else head[m] = i;
         tail[m] = i;
         if (m > maxm) maxm = m;
     }
     void remove(int m, int i) {
-        if (prev[i] >= 0) next[prev[i]] = next[i]; else head[m] = next[i];
-        if (next[i] >= 0) prev[next[i]] = prev[i]; else tail[m] = prev[i];
+        const int nx = p[i].next, pv = p[i].prev;
+        if (pv >= 0) p[pv].next = nx; else head[m] = nx;
+        if (nx >= 0) p[nx].prev = pv; else tail[m] = pv;
         while (maxm > 0 && head[maxm] < 0) --maxm;
     }
 };
@@ -73,42 +86,44 @@ void rs_first_pass_host(int n, const int *Si, const int *Sj, int *CF, const int 
 void rs_first_pass_host(int n, const int *Si, const int *Sj, const int *STi, const int *STj, int *CF,
                         const int *gia) {
     const int C_PT = 1, F_PT = -1, Z_PT = -2, SF_PT = -3, UNDEC = 0;
-    std::vector<int> measure(n);
-    int maxmeasure = 0;
-    for (int i = 0; i < n; ++i) {
-        measure[i] = STi[i + 1] - STi[i];
-        maxmeasure = std::max(maxmeasure, measure[i]);
-    }
-    Buckets B(n, maxmeasure + n + 2);
-    int num_left = 0;
+    Buckets B(n);
+    Point *P = B.p.data();
+    int maxmeasure = 0, num_left = 0;
     const int *rows = gia ? gia : Si;
-    for (int j = 0; j < n; ++j) {
-        if (rows[j + 1] - rows[j] == 0) {
-            CF[j] = SF_PT;
-            measure[j] = 0;
+    for (int i = 0; i < n; ++i) {
+        P[i].measure = STi[i + 1] - STi[i];
+        maxmeasure = std::max(maxmeasure, P[i].measure);
+        if (rows[i + 1] - rows[i] == 0) {
+            P[i].cf = SF_PT;
+            P[i].measure = 0;
         } else {
-            CF[j] = UNDEC;
+            P[i].cf = UNDEC;
             ++num_left;
         }
     }
+    B.init(maxmeasure);
+    // a point that an F point depends on: one measure up
+    auto raise = [&](int i) {
+        const int m = P[i].measure;
+        B.remove(m, i);
+        P[i].measure = m + 1;
+        B.enter(m + 1, i);
+    };
     for (int j = 0; j < n; ++j) {
-        const int m = measure[j];
-        if (CF[j] == SF_PT) continue;
-        if (m > 0) {
-            B.enter(m, j);
+        if (P[j].cf == SF_PT) continue;
+        if (P[j].measure > 0) {
+            B.enter(P[j].measure, j);
         } else {
-            CF[j] = Z_PT;
+            P[j].cf = Z_PT;
             for (int k = Si[j]; k < Si[j + 1]; ++k) {
                 const int nb = Sj[k];
-                if (CF[nb] != SF_PT) {
-                    if (nb < j) {
-                        int nm = measure[nb];
-                        if (nm > 0) B.remove(nm, nb);
-                        nm = ++measure[nb];
-                        B.enter(nm, nb);
-                    } else {
-                        ++measure[nb];
-                    }
+                if (P[nb].cf == SF_PT) continue;
+                if (nb < j) {
+                    if (P[nb].measure > 0) B.remove(P[nb].measure, nb);
+                    ++P[nb].measure;
+                    B.enter(P[nb].measure, nb);
+                } else {
+                    ++P[nb].measure;
                 }
             }
             --num_left;
@@ -116,48 +131,35 @@ void rs_first_pass_host(int n, const int *Si, const int *Sj, const int *STi, con
     }
     while (num_left > 0) {
         const int index = B.head[B.maxm];
-        CF[index] = C_PT;
-        const int m = measure[index];
-        measure[index] = 0;
+        P[index].cf = C_PT;
+        const int m = P[index].measure;
+        P[index].measure = 0;
         --num_left;
         B.remove(m, index);
         for (int k = STi[index]; k < STi[index + 1]; ++k) {
             const int nb = STj[k];
-            if (CF[nb] == UNDEC) {
-                CF[nb] = F_PT;
-                B.remove(measure[nb], nb);
-                --num_left;
-                for (int q = Si[nb]; q < Si[nb + 1]; ++q) {
-                    const int n2 = Sj[q];
-                    if (CF[n2] == UNDEC) {
-                        B.remove(measure[n2], n2);
-                        B.enter(++measure[n2], n2);
-                    }
-                }
-            }
+            if (P[nb].cf != UNDEC) continue;
+            P[nb].cf = F_PT;
+            B.remove(P[nb].measure, nb);
+            --num_left;
+            for (int q = Si[nb]; q < Si[nb + 1]; ++q)
+                if (P[Sj[q]].cf == UNDEC) raise(Sj[q]);
         }
         for (int k = Si[index]; k < Si[index + 1]; ++k) {
             const int nb = Sj[k];
-            if (CF[nb] == UNDEC) {
-                int mm = measure[nb];
-                B.remove(mm, nb);
-                measure[nb] = --mm;
-                if (mm > 0) {
-                    B.enter(mm, nb);
-                } else {
-                    CF[nb] = F_PT;
-                    --num_left;
-                    for (int q = Si[nb]; q < Si[nb + 1]; ++q) {
-                        const int n2 = Sj[q];
-                        if (CF[n2] == UNDEC) {
-                            B.remove(measure[n2], n2);
-                            B.enter(++measure[n2], n2);
-                        }
-                    }
-                }
+            if (P[nb].cf != UNDEC) continue;
+            B.remove(P[nb].measure, nb);
+            if (--P[nb].measure > 0) {
+                B.enter(P[nb].measure, nb);
+            } else {
+                P[nb].cf = F_PT;
+                --num_left;
+                for (int q = Si[nb]; q < Si[nb + 1]; ++q)
+                    if (P[Sj[q]].cf == UNDEC) raise(Sj[q]);
             }
         }
     }
+    for (int i = 0; i < n; ++i) CF[i] = P[i].cf;
 }
 
 void rs_first_pass_ranges(int n, const int *Si, const int *Sj, int range_rows, int *CF) {
