@@ -93,6 +93,11 @@ void bsr_decouple_rhs(int nb, int bs, int type, const double *coef, double *rhs,
 template <typename V, typename X>
 void bsr_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, int *err, cudaStream_t stream,
               bool staged = true);
+// y = A x for an FP32 x (16-byte aligned, widened before the products: the product with the FP64 vector of
+// the same values), which is also stored as ZT in Z[*i] (device pointers).
+template <typename ZT>
+void bsr_spmv_keep(const BsrView<double> &A, const float *x, double *y, ZT *const *Z, const int *i,
+                   cudaStream_t stream);
 
 // ---- blas1.cu --------------------------------------------------------------
 // Deterministic two-pass reductions: per-CTA partials into `partials`
