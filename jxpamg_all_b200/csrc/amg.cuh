@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "exact_sweep.cuh"
 #include "kernels.cuh"
 
 namespace jxcpr {
@@ -53,6 +54,8 @@ struct AmgLevel {
     DeviceCsr R;          // P^T, rows listing fine points ascending
     std::vector<int> cf;  // host copy of the C/F splitting (tests)
     Schedule fwd, bwd;    // Gauss-Seidel schedules
+    SweepStream sfwd, sbwd;  // exact order: the operator in schedule order, where the sweeps run from it
+    SweepStreamHost blk_fwd, blk_bwd;  // level 0, exact order: the block matrix's streams (host part)
     std::vector<int> chunk_order, chunk_seg;  // level 0 of the fast path: stage-2 chunk order (host)
     DevBuf<double> f, u;  // right-hand side and iterate of this level
 };
@@ -68,6 +71,7 @@ struct AmgParams {
     double jacobi_mean_row = 12.0;  // multicolour mode: levels with longer mean rows go straight to l1-Jacobi
     int rs_range_rows = 0;  // > 0: the coarsening's first pass runs on row ranges of this size (host threads)
     int rs_range_rows_coarse = 0;  // the same on the levels below the finest
+    int sweep_bs = 0;       // > 0 (exact order): level 0 also gets the streams of a block matrix of its pattern
     int stage2_chunk = 0;   // > 0 (fast path): level 0 also gets the stage-2 chunk order (build_chunk_order_host)
     // Optional per-level strength thresholds: called before level l is
     // coarsened with its operator; returns the threshold to use (learned model).
@@ -142,15 +146,16 @@ void permute_rows_bsr(const BsrView<double> &A, const int *perm, DeviceBsr &P, c
 // pass.
 void gs_sweep(const CsrView<double> &A, const Schedule &sch, const double *f, double *u, const int *rank,
               double *vt, int *err, cudaStream_t s);
-// Stage-2 block hybrid Gauss-Seidel (jxf_ParBSRHGSRelax) along `sch`; vt is
-// scratch (nb*bs) that receives the iterate at sweep start.
-void hgs_sweep(const BsrView<double> &A, const Schedule &sch, const double *b, double *x, const int *rank,
-               double *vt, double w, double omega, int *err, cudaStream_t s);
+// Stage-2 block hybrid Gauss-Seidel (jxf_ParBSRHGSRelax) along `sch`, from
+// `stream` where it is ready; vt is scratch (nb*bs) that receives the iterate at sweep start.
+void hgs_sweep(const BsrView<double> &A, const Schedule &sch, const SweepStream &stream, const double *b, double *x,
+               const int *rank, double *vt, double w, double omega, int *err, cudaStream_t s);
 // Stage-2 block hybrid symmetric Gauss-Seidel (jxf_ParBSRHSGSRelax, par_relax_bsr.c:579-1062): a
 // forward pass along `fwd`, then a backward pass along `bwd`.  vt: scratch (nb*bs); work: the CPR's
 // work vector (nb*bs, zero when created), of which only the first nb entries are refreshed from x,
 // as the reference does, and which feeds the res2 term of the weighted update.
-void hsgs_sweep(const BsrView<double> &A, const Schedule &fwd, const Schedule &bwd, const double *b, double *x,
-                double *vt, double *work, double w, double omega, int *err, cudaStream_t s);
+void hsgs_sweep(const BsrView<double> &A, const Schedule &fwd, const Schedule &bwd, const SweepStream &sfwd,
+                const SweepStream &sbwd, const double *b, double *x, double *vt, double *work, double w, double omega,
+                int *err, cudaStream_t s);
 
 }  // namespace jxcpr

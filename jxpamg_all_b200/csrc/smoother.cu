@@ -15,13 +15,16 @@
 //   with its Kahan-compensated block products (seq_bsr_matrix.c:841-872) and
 //   2x2 / 3x3 diagonal-block solves (:945-1100).
 //
-// Execution: one persistent cooperative kernel per sweep; groups are
-// separated by a grid barrier whose wait is bounded (a timeout raises the
-// error flag and every CTA leaves).  Small systems run in a single CTA with
-// __syncthreads between groups.
+// Execution: schedules of narrow groups are swept by one block from a stream
+// in schedule order (exact_sweep.cu).  The others (wide groups; patterns the
+// stream does not cover) run here: one persistent cooperative kernel per
+// sweep, groups separated by a grid barrier whose wait is bounded (a timeout
+// raises the error flag and every CTA leaves), or, for small systems, a single
+// CTA with __syncthreads between groups.
 #include <cooperative_groups.h>
 
 #include "amg.cuh"
+#include "block_ops.cuh"
 #include "common.cuh"
 #include "grid_sync.cuh"
 
@@ -81,94 +84,6 @@ __global__ void gs_sweep_block_kernel(int ngroups, const int *__restrict__ gptr,
 // ---------------------------------------------------------------------------
 // block hybrid Gauss-Seidel row update
 // ---------------------------------------------------------------------------
-template <int BS>
-__device__ __forceinline__ void blk_matvec_stable(double alpha, const double *__restrict__ mat, const double *v,
-                                                  double *ov) {
-    double tmp[BS];
-#pragma unroll
-    for (int j = 0; j < BS; ++j) tmp[j] = ov[j] * 1.0;
-#pragma unroll
-    for (int i = 0; i < BS; ++i) {
-        double sum = 0.0, c = 0.0;
-#pragma unroll
-        for (int j = 0; j < BS; ++j) {
-            const double y = mat[i * BS + j] * v[j] - c;
-            const double t = sum + y;
-            c = (t - sum) - y;
-            sum = t;
-        }
-        tmp[i] += alpha * sum;
-        ov[i] = tmp[i];
-    }
-}
-
-template <int BS>
-__device__ __forceinline__ void blk_inv_matvec(const double *__restrict__ mat, const double *v, double *ov) {
-    if (BS == 2) {
-        const double a11 = mat[0], a12 = mat[1], a21 = mat[2], a22 = mat[3];
-        const double det = a11 * a22 - a12 * a21;
-        if (fabs(det) < 1e-12 * (fabs(a11 * a22) + fabs(a12 * a21))) {
-            ov[0] = v[0] / (a11 + 1e-12);
-            ov[1] = v[1] / (a22 + 1e-12);
-            return;
-        }
-        const double inv_det = 1.0 / det;
-        const double b1 = v[0], b2 = v[1];
-        ov[0] = (a22 * b1 - a12 * b2) * inv_det;
-        ov[1] = (-a21 * b1 + a11 * b2) * inv_det;
-        return;
-    }
-    double m[9], x[3], o[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < 9; ++q) m[q] = mat[q];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) x[q] = v[q];
-    const int n = 3;
-    for (int i = 0; i < n; ++i) {
-        int mr = i;
-        double mv = fabs(m[i * n + i]);
-        for (int k = i + 1; k < n; ++k)
-            if (fabs(m[k * n + i]) > mv) {
-                mv = fabs(m[k * n + i]);
-                mr = k;
-            }
-        if (mv < 1e-15) {
-            for (int j = 0; j < n; ++j) {
-                const double d = m[j * n + j];
-                o[j] = (fabs(d) > 1e-12) ? x[j] / d : 0.0;
-            }
-            break;
-        }
-        if (mr != i) {
-            for (int j = 0; j < n; ++j) {
-                const double t = m[i * n + j];
-                m[i * n + j] = m[mr * n + j];
-                m[mr * n + j] = t;
-            }
-            const double t = x[i];
-            x[i] = x[mr];
-            x[mr] = t;
-        }
-        const double pivot = m[i * n + i];
-        for (int k = i + 1; k < n; ++k) {
-            const double fct = m[k * n + i] / pivot;
-            m[k * n + i] = fct;
-            for (int j = i + 1; j < n; ++j) m[k * n + j] -= fct * m[i * n + j];
-        }
-    }
-    for (int i = 0; i < n; ++i) {
-        o[i] = x[i];
-        for (int j = 0; j < i; ++j) o[i] -= m[i * n + j] * o[j];
-    }
-    for (int i = n - 1; i >= 0; --i) {
-        for (int j = i + 1; j < n; ++j) o[i] -= m[i * n + j] * o[j];
-        const double d = m[i * n + i];
-        if (fabs(d) > 1e-15) o[i] /= d; else o[i] = 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) ov[q] = o[q];
-}
-
 // vt: the iterate at the start of the pass (read for neighbours not yet
 // updated in it); vt2: the vector of the res2 term (vt for HGS, the CPR's work
 // vector for HSGS).
@@ -354,21 +269,31 @@ int plain_weights(double w, double omega) {
 }
 }  // namespace
 
-void hgs_sweep(const BsrView<double> &A, const Schedule &sch, const double *b, double *x, const int *rank,
-               double *vt, double w, double omega, int *err, cudaStream_t s) {
+void hgs_sweep(const BsrView<double> &A, const Schedule &sch, const SweepStream &stream, const double *b, double *x,
+               const int *rank, double *vt, double w, double omega, int *err, cudaStream_t s) {
     const int nb = A.nb;
     if (nb == 0 || sch.ngroups == 0) return;
+    if (stream.ready()) {
+        hgs_stream(A, stream, b, x, x, w, omega, plain_weights(w, omega), err, s);
+        return;
+    }
     JX_CUDA(cudaMemcpyAsync(vt, x, sizeof(double) * nb * A.bs, cudaMemcpyDeviceToDevice, s));
     hgs_pass(A, sch, b, x, rank, vt, vt, w, omega, plain_weights(w, omega), err, s);
 }
 
-void hsgs_sweep(const BsrView<double> &A, const Schedule &fwd, const Schedule &bwd, const double *b, double *x,
-                double *vt, double *work, double w, double omega, int *err, cudaStream_t s) {
+void hsgs_sweep(const BsrView<double> &A, const Schedule &fwd, const Schedule &bwd, const SweepStream &sfwd,
+                const SweepStream &sbwd, const double *b, double *x, double *vt, double *work, double w, double omega,
+                int *err, cudaStream_t s) {
     const int nb = A.nb;
     if (nb == 0 || fwd.ngroups == 0 || bwd.ngroups == 0) return;
     const int plain = plain_weights(w, omega);
     // the reference refreshes only the first nb (block-row count) entries of its work vector
     if (!plain) JX_CUDA(cudaMemcpyAsync(work, x, sizeof(double) * nb, cudaMemcpyDeviceToDevice, s));
+    if (sfwd.ready() && sbwd.ready()) {
+        hgs_stream(A, sfwd, b, x, work, w, omega, plain, err, s);
+        hgs_stream(A, sbwd, b, x, work, w, omega, plain, err, s);
+        return;
+    }
     JX_CUDA(cudaMemcpyAsync(vt, x, sizeof(double) * nb * A.bs, cudaMemcpyDeviceToDevice, s));
     hgs_pass(A, fwd, b, x, fwd.rank.get(), vt, work, w, omega, plain, err, s);
     JX_CUDA(cudaMemcpyAsync(vt, x, sizeof(double) * nb * A.bs, cudaMemcpyDeviceToDevice, s));

@@ -35,6 +35,7 @@ void CprPrecond::setup(const BsrView<double> &A_, cudaStream_t s) {
     amg.prm.max_colors = prm.max_colors;
     amg.prm.jacobi_mean_row = prm.jacobi_mean_row;
     amg.prm.stage2_chunk = fast_path ? prm.stage2_chunk : 0;
+    amg.prm.sweep_bs = !fast_path && (prm.stage2_solver_type == 2 || prm.stage2_solver_type == 3) ? A.bs : 0;
     amg.prm.rs_range_rows = fast_path ? prm.rs_range_rows : 0;
     amg.prm.rs_range_rows_coarse = fast_path ? (prm.rs_range_rows_coarse > 0 ? prm.rs_range_rows_coarse
                                                                               : prm.rs_range_rows) : 0;
@@ -60,6 +61,15 @@ void CprPrecond::setup(const BsrView<double> &A_, cudaStream_t s) {
     bsr_pressure_csr(A, prm.pressure_index, Ap, s);
     amg_setup(amg, std::move(Ap), s);
     amg.prm.theta_for_level = nullptr;
+    blk_fwd = SweepStream();
+    blk_bwd = SweepStream();
+    if (amg.prm.sweep_bs > 0 && !amg.levels[0]->blk_fwd.desc.empty()) {
+        AmgLevel &L0 = *amg.levels[0];
+        upload_sweep_stream(L0.blk_fwd, A.bs, A.ia, A.a, blk_fwd, s);
+        if (prm.stage2_solver_type == 3) upload_sweep_stream(L0.blk_bwd, A.bs, A.ia, A.a, blk_bwd, s);
+        L0.blk_fwd = SweepStreamHost();
+        L0.blk_bwd = SweepStreamHost();
+    }
     if (fast_path) {
         CprConfig cfg;
         cfg.pressure_index = prm.pressure_index;
@@ -173,11 +183,11 @@ void CprPrecond::stage2_sweep(const double *r, double *z, cudaStream_t s) {
     }
     const AmgLevel &L0 = *amg.levels[0];
     if (prm.stage2_solver_type == 3) {
-        hsgs_sweep(A, L0.fwd, L0.bwd, r, z, vt.get(), hsgs_work.get(), prm.stage2_relax_weight, prm.stage2_omega,
+        hsgs_sweep(A, L0.fwd, L0.bwd, blk_fwd, blk_bwd, r, z, vt.get(), hsgs_work.get(), prm.stage2_relax_weight, prm.stage2_omega,
                    amg.err.get(), s);
         return;
     }
-    hgs_sweep(A, L0.fwd, r, z, L0.fwd.rank.get(), vt.get(), prm.stage2_relax_weight, prm.stage2_omega,
+    hgs_sweep(A, L0.fwd, blk_fwd, r, z, L0.fwd.rank.get(), vt.get(), prm.stage2_relax_weight, prm.stage2_omega,
               amg.err.get(), s);
 }
 
@@ -344,7 +354,7 @@ void Gmres::setup(int n_, cudaStream_t s) {
     r.alloc(n > 0 ? n : 1);
     w.alloc(n > 0 ? n : 1);
     cgs_blocks = std::max(1, std::min(4 * sm_count(), div_up(n > 0 ? n : 1, kCgsThreads)));
-    partials.alloc(std::max<size_t>(reduce_partials() + 8, (size_t)cgs_blocks * kCgsMax));
+    partials.alloc(std::max<size_t>(2 * (reduce_partials() + 8), (size_t)cgs_blocks * kCgsMax));  // two passes' partials
     scal.alloc(prm.k_dim + 8);
     std::vector<const double *> ptrs;
     for (auto &v : p) ptrs.push_back(v.get());

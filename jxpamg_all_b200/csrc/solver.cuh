@@ -118,6 +118,7 @@ struct CprPrecond {
     SolverParams prm;
     BsrView<double> A;  // decoupled system matrix (owned by the solver)
     Amg amg;
+    SweepStream blk_fwd, blk_bwd;  // exact order: the block matrix in schedule order
     std::unique_ptr<FastCprBase> fast;  // smoother_order 1: throughput / mixed-precision preconditioner
     bool probe_pending = false;  // learned mode: the plain-vs-learned probe runs after GMRES setup
     std::unique_ptr<Bilu> bilu;         // stage2_solver_type 5
