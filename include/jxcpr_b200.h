@@ -168,7 +168,9 @@ JXCPR_API int jxcpr_dense_inverse_dev(int n, const double *a, double *ainv, void
  *         norm, rotation, residual and x in FP64), selective_reorth (0; 1
  *         with graph_gmres: the second classical Gram-Schmidt pass only when
  *         the first removed more than half of ||w||^2), orthog (0 modified, 1 one-pass classical
- *         Gram-Schmidt), autotune (1; 2 shared per shape class), stage2_lanes
+ *         Gram-Schmidt), autotune (1: level operators of 200,000 rows and
+ *         more are timed in each layout at setup, smaller ones take theirs by
+ *         size; 2 timings shared per shape class), stage2_lanes
  *         (4: CSR stage 2 without autotuning), stage2_chunk (4: stage 2 visits
  *         chunks of this many consecutive block rows in natural order, the
  *         chunks coloured for parallelism; 8 or 16 also accepted; 0: the

@@ -80,8 +80,12 @@ struct FastLevel {
     int smoother_cfg = FS_L1_JACOBI, smoother_plain = FS_L1_JACOBI;  // configured / plain settings
     LevelMat A;          // colour classes as segments (FS_COLOR_GS) or one segment
     const int *src_ia = nullptr, *src_ja = nullptr;  // the hierarchy's CSR operator's pattern (not owned)
-    int last_color = -1;
     LevelMat P, R;       // interpolation from level+1 / restriction to it
+    // Level 0 with multicolour GS: smoothing ends with colour class 0, so its residual there is zero, and the
+    // next smoothing starts with that class, so it overwrites the correction there.  The residual and the
+    // interpolation run on the other classes only (P in colour order), R lists no columns of class 0.
+    bool skip_class0 = false;
+    DevBuf<TX> dinv0;    // level 0 with multicolour GS: 1/a_ii on class 0, 0 elsewhere
     DevBuf<TX> dinv;     // 1/a_ii (GS, Chebyshev); 0 skips the row
     DevBuf<TX> dinv_l1;  // 1/sum_j |a_ij| (l1-Jacobi)
     double cheb[3] = {0, 0, 0};  // p(t) = c0 + c1 t + c2 t^2
@@ -120,6 +124,10 @@ struct FastCprBase {
     // The application's kernels queued on s, never through the private graph:
     // for callers that capture the application into a graph of their own.
     virtual void apply_enqueue(const double *r, double *z, cudaStream_t s) = 0;
+    // The application's kernels on basis vector V[*i] (one of v32 / v64: device arrays of vectors), queued on
+    // s, its FP32 result left in the returned vector; nullptr, with nothing queued, where the result is FP64.
+    virtual const float *apply_enqueue_basis(const float *const *v32, const double *const *v64, const int *i,
+                                             cudaStream_t s) = 0;
     virtual void vcycle(const double *fp, double *up, cudaStream_t s) = 0;  // FP64 pressure in/out
     virtual void stage2_sweep(const double *r, double *z, cudaStream_t s) = 0;
     virtual int num_levels() const = 0;

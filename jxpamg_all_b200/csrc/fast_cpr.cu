@@ -50,21 +50,31 @@ void launch_csr(const LevelMat &M, const TV *a, const Op &op, int r0, int r1, cu
                f, op, r0, r1);
 }
 
+template <typename TX, int P, typename TV, class Op>
+void launch_sell(const LevelMat &M, const TV *a, const Op &op, int r0, int r1, cudaStream_t s) {
+    fk::SellFmt<TV, P> f{M.sp.get(), M.ja.get(), a, M.bscale.get(), M.rows.get()};
+    launch_dep(fk::row_kernel<fk::SellFmt<TV, P>, Op, TX>, dim3(div_up((long long)(r1 - r0) * P, kThreads)),
+               dim3(kThreads), s, f, op, r0, r1);
+}
+
 template <typename TX, class Op>
 void launch_rows(const LevelMat &M, const Op &op, int r0, int r1, cudaStream_t s) {
     if (r1 <= r0) return;
     with_values<TX>(M, [&](auto a) {
         using TV = typename std::remove_cv<typename std::remove_pointer<decltype(a)>::type>::type;
-        if (M.sell == 2) {
-            fk::SellFmt<TV, 2> f{M.sp.get(), M.ja.get(), a, M.bscale.get(), M.rows.get()};
-            launch_dep(fk::row_kernel<fk::SellFmt<TV, 2>, Op, TX>, dim3(div_up((long long)(r1 - r0) * 2, kThreads)),
-                       dim3(kThreads), s, f, op, r0, r1);
-            return;
-        }
         if (M.sell) {
-            fk::SellFmt<TV> f{M.sp.get(), M.ja.get(), a, M.bscale.get(), M.rows.get()};
-            launch_dep(fk::row_kernel<fk::SellFmt<TV>, Op, TX>, dim3(div_up(r1 - r0, kThreads)), dim3(kThreads), s,
-                       f, op, r0, r1);
+            if constexpr (std::is_same<TV, __nv_bfloat16>::value) {
+                launch_sell<TX, 1>(M, a, op, r0, r1, s);
+            } else {
+                switch (M.sell) {
+                    case 1: launch_sell<TX, 1>(M, a, op, r0, r1, s); break;
+                    case 2: launch_sell<TX, 2>(M, a, op, r0, r1, s); break;
+                    case 4: launch_sell<TX, 4>(M, a, op, r0, r1, s); break;
+                    case 8: launch_sell<TX, 8>(M, a, op, r0, r1, s); break;
+                    case 16: launch_sell<TX, 16>(M, a, op, r0, r1, s); break;
+                    default: launch_sell<TX, 32>(M, a, op, r0, r1, s); break;
+                }
+            }
             return;
         }
         switch (M.lanes) {
@@ -192,7 +202,7 @@ void build_level_mat(int n, int m, long long nnz, int E, const int *ia, const in
                      int sell, const std::vector<int> &order, const std::vector<int> &seg, const int *order_dev,
                      LevelMat &M, cudaStream_t s) {
     // sell: 0 CSR, 1 sliced ELL, 2 sliced ELL with two lanes per row (E = 1, FP32 / FP64 values)
-    if (sell == 2 && (E != 1 || kind == VAL_BF16)) sell = 1;
+    if (sell > 1 && (E != 1 || kind == VAL_BF16)) sell = 1;
     M.n = n;
     M.m = m;
     M.nnz = nnz;
@@ -221,18 +231,18 @@ void build_level_mat(int n, int m, long long nnz, int E, const int *ia, const in
         M.sp.upload(sp.data(), sp.size(), s);
         M.ja.alloc(slots > 0 ? slots : 1);
         const long long nv = (slots > 0 ? slots : 1) * E;
-        if (sell == 2) {
-            const long long lanes = (long long)M.nstored * 2;
+        if (sell > 1) {
+            const long long lanes = (long long)M.nstored * 32;  // a warp per stored row
             if (kind == VAL_F64) {
                 M.a64.alloc(nv);
                 if (lanes)
                     fk::sell_fill_lanes<double><<<div_up(lanes, kThreads), kThreads, 0, s>>>(
-                        M.nstored, 2, M.rows.get(), M.sp.get(), ia, ja, a, M.ja.get(), M.a64.get(), 0);
+                        M.nstored, sell, M.rows.get(), M.sp.get(), ia, ja, a, M.ja.get(), M.a64.get(), 0);
             } else {
                 M.a32.alloc(nv);
                 if (lanes)
                     fk::sell_fill_lanes<float><<<div_up(lanes, kThreads), kThreads, 0, s>>>(
-                        M.nstored, 2, M.rows.get(), M.sp.get(), ia, ja, a, M.ja.get(), M.a32.get(), 1);
+                        M.nstored, sell, M.rows.get(), M.sp.get(), ia, ja, a, M.ja.get(), M.a32.get(), 1);
             }
             JX_LAUNCH_CHECK();
         } else if (kind == VAL_F64) {
@@ -390,7 +400,7 @@ double time_pass(const LevelMat &M, const TX *x, TX *y, cudaStream_t s) {
 }
 
 std::string layout_name(const LevelMat &M) {
-    return M.sell == 2 ? std::string("sell/2") : M.sell ? std::string("sell") : ("csr/" + std::to_string(M.lanes));
+    return M.sell > 1 ? "sell/" + std::to_string(M.sell) : M.sell ? std::string("sell") : ("csr/" + std::to_string(M.lanes));
 }
 
 // Layout choices of earlier setups, keyed by operator role, shape and storage:
@@ -443,9 +453,36 @@ std::string tune_key(const char *name, int n, long long nnz, int kind, int E, in
     return k;
 }
 
-// Builds a scalar operator in the layout that runs fastest here: CSR with
-// 1..32 lanes per row (the candidates around the mean row length), or sliced
-// ELL (operators with >= 2048 rows).
+// Operators with fewer rows take their layout by size.  Their passes run 2 to 8 us inside a solve's graph;
+// timed one by one from the host they all read as the 5 us of a launch, and the timing picked at random.
+constexpr int kTuneRows = 200000;
+
+// The sliced-ELL lanes per row for n rows of mean length `mean` (0: CSR).  The cost of a pass
+// with P lanes, fitted to passes timed in graphs (us, 1,110 to 128,778 rows of 20 to 228 entries, P = 1 to 32):
+// a chain of batches of eight slots (0.9 each) and the lanes' own cost (0.9 per 100,000).  It picks the
+// fastest P or one within 8 % of it at every measured size, e.g. rows x entries -> us of the picked layout /
+// of the one the timing had picked: 5,340 x 88 FP32 2.4 / 3.1, 23,039 x 138 6.2 / 7.4, 4,102 x 228 2.6 / 3.3.
+// Many short rows (the finest level, transfers) take one lane each, FP64 in sliced ELL (145,297 x 6.9: 2.8
+// against 3.7 in CSR), FP32 in CSR (1,122,000 x 6.9: 14.6 against 19.1; 264,000: the same).  Fewer than 512
+// rows are a warp or two in any layout and keep CSR.
+template <typename TX>
+int pick_layout(int n, double mean) {
+    if (n < 512) return 0;
+    if (mean <= 10.0 && n >= 50000) return sizeof(TX) == 8 ? 1 : 0;
+    int best = 1;
+    double cost = 1e30;
+    for (int P = 1; P <= 32; P *= 2) {
+        const double c = 0.9 * ceil(std::max(mean, 1.0) / (P * (double)fk::SellFmt<TX>::NB)) + 0.9e-5 * (double)n * P;
+        if (c < cost) {
+            cost = c;
+            best = P;
+        }
+    }
+    return best;
+}
+
+// Builds a scalar operator: below kTuneRows rows in pick_layout's layout, above in the one that runs fastest
+// here: CSR with 1..32 lanes per row (the candidates around the mean row length), or sliced ELL.
 template <typename TX>
 void build_tuned(const char *name, int n, int m, long long nnz, const int *ia, const int *ja, const double *a,
                  int kind, const std::vector<int> &order, const std::vector<int> &seg, const int *order_dev,
@@ -459,6 +496,16 @@ void build_tuned(const char *name, int n, int m, long long nnz, const int *ia, c
                      layout_name(M).c_str());
             log.emplace_back(line);
         }
+        return;
+    }
+    if (kind != VAL_BF16 && n < kTuneRows) {
+        const int sell = pick_layout<TX>(n, (double)nnz / n);
+        build_level_mat(n, m, nnz, 1, ia, ja, a, kind, sell, order, seg, order_dev, M, s);
+        if (!sell && n >= 512) M.lanes = 1;
+        char line[200];
+        snprintf(line, sizeof line, "%s rows %d mean %.1f layout %s (by size)", name, n, (double)nnz / n,
+                 layout_name(M).c_str());
+        log.emplace_back(line);
         return;
     }
     const std::string key = tune_key(name, n, nnz, kind, 1, opt.autotune);
@@ -579,7 +626,7 @@ __global__ void unpack_csr_kernel(int n, const int *__restrict__ perm, const int
 }
 
 template <typename TX>
-__global__ void add_kernel(int n, TX *__restrict__ u, const TX *__restrict__ c) {
+__global__ void add_kernel(int n, TX *u, const TX *c) {
     grid_dep_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) u[i] += c[i];
@@ -615,26 +662,6 @@ void chebyshev3_coefficients(double lo, double hi, double c[3]) {
     c[2] = -n3 / n0;
 }
 
-// One power step's scalars on the device: lam = sqrt(<y,y> / <x,x>) and the scale 1 / ||y|| of the
-// next iterate (the correctly rounded FP64 operations the host would do), or the stop flag once a
-// norm is not positive (lam keeps its last value).  st = {lam, scale, stop}.
-__global__ void power_scalars_kernel(const double *__restrict__ nrm, double *st) {
-    if (st[2] != 0.0) return;
-    const double yy = nrm[0], xx = nrm[1];
-    if (!(yy > 0.0) || !(xx > 0.0)) {
-        st[2] = 1.0;
-        return;
-    }
-    st[0] = sqrt(yy / xx);
-    st[1] = 1.0 / sqrt(yy);
-}
-__global__ void power_scale_kernel(int n, const double *__restrict__ st, double *__restrict__ y) {
-    if (st[2] != 0.0) return;
-    const double a = st[1];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = a * y[i];
-}
-
 // lambda_max(D^-1 A) by `iters` power steps from x = 1, with the host reading the result once.
 // iters2 > iters: the power steps go on to iters2 and *lam2 receives that estimate too (the same
 // sequence of iterates, so each value equals a separate run of that many steps).
@@ -644,7 +671,9 @@ double estimate_lambda_max(const CsrView<double> &A, int iters, cudaStream_t s, 
         if (lam2) *lam2 = 1.0;
         return 1.0;
     }
-    DevBuf<double> dinv(n), x(n), y(n), partials(reduce_partials() + 8), nrm(2), st(3);
+    const int V = lanes_for((double)A.nnz / n);
+    const int grid = std::max(1, std::min(2 * sm_count(), div_up((long long)n * V, fk::kPowerThreads)));
+    DevBuf<double> dinv(n), x(n), y(n), part(2 * (size_t)grid), st(3);
     fk::dinv_diag<double><<<div_up(n, kThreads), kThreads, 0, s>>>(n, A.ia, A.ja, A.a, dinv.get());
     JX_LAUNCH_CHECK();
     fill_dev(n, 1.0, x.get(), s);
@@ -655,13 +684,11 @@ double estimate_lambda_max(const CsrView<double> &A, int iters, cudaStream_t s, 
     for (int it = 0; it < total; ++it) {
         if (it == iters)
             JX_CUDA(cudaMemcpyAsync(at_iters.get(), st.get(), sizeof(double), cudaMemcpyDeviceToDevice, s));
-        fk::dinv_a_x<<<div_up(n, kThreads), kThreads, 0, s>>>(n, A.ia, A.ja, A.a, dinv.get(), x.get(), y.get());
+        auto step = V >= 32 ? fk::power_step<32> : V >= 16 ? fk::power_step<16> : V >= 8 ? fk::power_step<8>
+                  : V >= 4 ? fk::power_step<4> : V >= 2 ? fk::power_step<2> : fk::power_step<1>;
+        step<<<grid, fk::kPowerThreads, 0, s>>>(n, A.ia, A.ja, A.a, dinv.get(), x.get(), st.get(), y.get(), part.get());
         JX_LAUNCH_CHECK();
-        dot_dev(n, y.get(), y.get(), partials.get(), nrm.get(), s);
-        dot_dev(n, x.get(), x.get(), partials.get(), nrm.get() + 1, s);
-        power_scalars_kernel<<<1, 1, 0, s>>>(nrm.get(), st.get());
-        JX_LAUNCH_CHECK();
-        power_scale_kernel<<<div_up(n, kThreads), kThreads, 0, s>>>(n, st.get(), y.get());
+        fk::power_scalars<<<1, 64, 0, s>>>(grid, part.get(), st.get());
         JX_LAUNCH_CHECK();
         std::swap(x.p, y.p);
     }
@@ -715,48 +742,74 @@ struct FastCpr final : FastCprBase {
         }
     }
 
+    // What the kernels around a smoothing take over: its first step from zero (the first colour class, or the
+    // step without neighbours) is done already; on level 0 the last passes also write the prolongation (z64 or
+    // z32).
+    struct Ends {
+        bool first_done = false;
+        double *z64 = nullptr;
+        float *z32 = nullptr;
+    };
+
     // ---- level operations ----------------------------------------------------
-    void smooth(FastLevel<TX> &L, const TX *f, TX *u, bool zero, cudaStream_t s) {
+    void smooth(FastLevel<TX> &L, const TX *f, TX *u, bool zero, cudaStream_t s, const Ends &E = Ends()) {
         if (L.n == 0) return;
         const LevelMat &M = L.A;
         if (L.smoother == FS_COLOR_GS) {
             const int ncol = (int)M.seg.size() - 1;
-            L.last_color = -1;
-            for (int rep = 0; rep < 4; ++rep) {  // two symmetric GS applications: fwd, bwd, fwd, bwd
-                const bool backward = rep & 1;
+            std::vector<int> pass;
+            for (int rep = 0; rep < 4; ++rep)  // two symmetric GS applications: fwd, bwd, fwd, bwd
                 for (int g = 0; g < ncol; ++g) {
-                    const int c = backward ? ncol - 1 - g : g;
-                    if (c == L.last_color) continue;  // recomputing the last class changes nothing
-                    L.last_color = c;
-                    fk::OpGs<TX> op{f, L.dinv.get(), u, zero ? 1 : 0};
-                    launch_rows<TX>(M, op, M.seg[c], M.seg[c + 1], s);
-                    zero = false;
+                    const int c = (rep & 1) ? ncol - 1 - g : g;
+                    if (!pass.empty() && pass.back() == c) continue;  // recomputing the last class changes nothing
+                    pass.push_back(c);
                 }
+            for (size_t q = 0; q < pass.size(); ++q) {
+                const int c = pass[q];
+                if (zero && q == 0) {  // class 0 alone; the others start from 0
+                    if (E.first_done) continue;
+                    launch_dep(fk::gs_first_class<TX>, dim3(div_up(M.nstored, kThreads)), dim3(kThreads), s,
+                               M.nstored, M.seg[1], M.sell ? M.rows.get() : M.perm, f, L.dinv.get(), u);
+                    JX_LAUNCH_CHECK();
+                    continue;
+                }
+                const fk::OpGs<TX> op{f, L.dinv.get(), u};
+                const bool last = std::find(pass.begin() + q + 1, pass.end(), c) == pass.end();
+                if (last && E.z64)
+                    launch_rows<TX>(M, fk::OpGsZ<TX, double>{op, E.z64, bs, cfg.pressure_index}, M.seg[c], M.seg[c + 1], s);
+                else if (last && E.z32)
+                    launch_rows<TX>(M, fk::OpGsZ<TX, float>{op, E.z32, bs, cfg.pressure_index}, M.seg[c], M.seg[c + 1], s);
+                else
+                    launch_rows<TX>(M, op, M.seg[c], M.seg[c + 1], s);
             }
         } else if (L.smoother == FS_L1_JACOBI) {
             for (int rep = 0; rep < 2; ++rep) {  // 2 x (u -> tmp -> u)
-                fk::OpJacobi<TX> a{f, L.dinv_l1.get(), u, L.z.get(), zero ? 1 : 0};
-                launch_rows<TX>(M, a, 0, M.nstored, s);
+                if (!(zero && E.first_done)) {
+                    fk::OpJacobi<TX> a{f, L.dinv_l1.get(), u, L.z.get(), zero ? 1 : 0};
+                    launch_rows<TX>(M, a, 0, M.nstored, s);
+                }
                 fk::OpJacobi<TX> b{f, L.dinv_l1.get(), L.z.get(), u, 0};
                 launch_rows<TX>(M, b, 0, M.nstored, s);
                 zero = false;
             }
         } else {
-            fk::OpCheb<TX> c0{0, zero ? 1 : 0, (TX)L.cheb[2], f, L.dinv.get(), nullptr, u, L.z.get(), L.y1.get()};
-            launch_rows<TX>(M, c0, 0, M.nstored, s);
+            if (!(zero && E.first_done)) {
+                fk::OpCheb<TX> c0{0, zero ? 1 : 0, (TX)L.cheb[2], f, L.dinv.get(), nullptr, u, L.z.get(), L.y1.get()};
+                launch_rows<TX>(M, c0, 0, M.nstored, s);
+            }
             fk::OpCheb<TX> c1{1, 0, (TX)L.cheb[1], f, L.dinv.get(), L.y1.get(), u, L.z.get(), L.y2.get()};
             launch_rows<TX>(M, c1, 0, M.nstored, s);
             fk::OpCheb<TX> c2{2, zero ? 1 : 0, (TX)L.cheb[0], f, L.dinv.get(), L.y2.get(), u, L.z.get(), nullptr};
             launch_rows<TX>(M, c2, 0, M.nstored, s);
         }
     }
-    void residual(FastLevel<TX> &L, const TX *f, const TX *u, TX *r, cudaStream_t s) {
+    void residual(FastLevel<TX> &L, const TX *f, const TX *u, TX *r, cudaStream_t s, int r0 = 0) {
         fk::OpResid<TX> op{f, u, r};
-        launch_rows<TX>(L.A, op, 0, L.A.nstored, s);
+        launch_rows<TX>(L.A, op, r0, L.A.nstored, s);
     }
-    void spmv(const LevelMat &M, const TX *x, bool beta_one, TX *y, cudaStream_t s) {
+    void spmv(const LevelMat &M, const TX *x, bool beta_one, TX *y, cudaStream_t s, int r0 = 0) {
         fk::OpSpmv<TX> op{x, y, beta_one ? 1 : 0};
-        launch_rows<TX>(M, op, 0, M.nstored, s);
+        launch_rows<TX>(M, op, r0, M.nstored, s);
     }
     void coarse(const TX *f, TX *u, cudaStream_t s) {
         if (nc == 0) return;
@@ -918,7 +971,7 @@ struct FastCpr final : FastCprBase {
     }
 
     // u0 = V-cycle(f0) from a zero initial guess
-    void vcycle_tx(const TX *f0, TX *u0, cudaStream_t s) {
+    void vcycle_tx(const TX *f0, TX *u0, cudaStream_t s, const Ends &E = Ends()) {
         const int L = (int)lv.size();
         auto F = [&](int l) -> const TX * { return l == 0 ? f0 : lv[l]->f.get(); };
         auto U = [&](int l) -> TX * { return l == 0 ? u0 : lv[l]->u.get(); };
@@ -929,10 +982,25 @@ struct FastCpr final : FastCprBase {
         const int top = tail_first > 0 ? tail_first : L - 1;  // levels above the fused ones
         for (int l = 0; l < top; ++l) {
             FastLevel<TX> &Lv = *lv[l];
-            if (Lv.smoother == FS_COLOR_GS && Lv.n) JX_CUDA(cudaMemsetAsync(U(l), 0, sizeof(TX) * Lv.n, s));
-            smooth(Lv, F(l), U(l), true, s);
-            residual(Lv, F(l), U(l), Lv.r.get(), s);
-            spmv(Lv.R, Lv.r.get(), false, lv[l + 1]->f.get(), s);
+            Ends pre;
+            pre.first_done = l == 0 ? E.first_done : lv[l]->smoother != FS_COLOR_GS;
+            smooth(Lv, F(l), U(l), true, s, pre);
+            const int r0 = Lv.skip_class0 ? Lv.A.seg[1] : 0;
+            residual(Lv, F(l), U(l), Lv.r.get(), s, r0);
+            if (r0 > 0 && F(l) == Lv.r.get()) {  // a right-hand side that the residual replaces: class 0 too
+                launch_dep(fk::zero_rows<TX>, dim3(div_up(r0, kThreads)), dim3(kThreads), s, r0,
+                           Lv.A.sell ? Lv.A.rows.get() : Lv.A.perm, Lv.r.get());
+                JX_LAUNCH_CHECK();
+            }
+            FastLevel<TX> &Nx = *lv[l + 1];
+            if (l + 1 < top && Nx.smoother != FS_COLOR_GS) {
+                const bool cheb = Nx.smoother == FS_CHEB;
+                const fk::OpRestrict<TX> op{Lv.r.get(), cheb ? Nx.dinv.get() : Nx.dinv_l1.get(), Nx.f.get(), Nx.z.get(),
+                                            cheb ? Nx.y1.get() : nullptr, (TX)Nx.cheb[2]};
+                launch_rows<TX>(Lv.R, op, 0, Lv.R.nstored, s);
+            } else {
+                spmv(Lv.R, Lv.r.get(), false, Nx.f.get(), s);
+            }
         }
         if (tail_first > 0)
             launch_tail(s);
@@ -940,8 +1008,8 @@ struct FastCpr final : FastCprBase {
             coarse(F(L - 1), U(L - 1), s);
         for (int l = top - 1; l >= 0; --l) {
             FastLevel<TX> &Lv = *lv[l];
-            spmv(Lv.P, U(l + 1), true, U(l), s);
-            smooth(Lv, F(l), U(l), false, s);
+            spmv(Lv.P, U(l + 1), true, U(l), s, Lv.skip_class0 ? Lv.P.seg[1] : 0);
+            smooth(Lv, F(l), U(l), false, s, l == 0 ? E : Ends());
         }
     }
 
@@ -1029,8 +1097,10 @@ struct FastCpr final : FastCprBase {
             }
             const int grid = div_up(r1 - r0, kThreads);
 #define JX_HGS_CHUNK(BSV, CHV)                                                                              \
-    launch_dep(fk::hgs_chunk<BSV, CHV, TV, TAC, TXV>, dim3(grid), dim3(kThreads), s, r0, r1, M.sp.get(),     \
-               reinterpret_cast<const unsigned *>(M.ja.get()), a, M.rows.get(), r, z, vtp, w, om, plain, so.save)
+    launch_dep(grid <= sm_count() ? fk::hgs_chunk<BSV, CHV, TV, TAC, TXV, true>                               \
+                                  : fk::hgs_chunk<BSV, CHV, TV, TAC, TXV, false>,                             \
+               dim3(grid), dim3(kThreads), s, r0, r1, M.sp.get(), reinterpret_cast<const unsigned *>(M.ja.get()), a, \
+               M.rows.get(), r, z, vtp, w, om, plain, so.save)
             if (bs == 2) {
                 if (M.chunk == 4) JX_HGS_CHUNK(2, 4);
                 else if (M.chunk == 16) JX_HGS_CHUNK(2, 16);
@@ -1108,21 +1178,25 @@ struct FastCpr final : FastCprBase {
 
     void apply_enqueue(const double *r, double *z, cudaStream_t s) override { apply_direct(r, z, s); }
 
-    void apply_direct(const double *r, double *z, cudaStream_t s) {
-        DepLaunchScope dep(opt.dep_launch);
+    bool stage2_on() const { return cfg.stage2_solver_type == 2 && cfg.stage2_maxit > 0; }
+    // FP32 result: stage 2 runs on FP32 copies of r and z (r32, z32)
+    bool native_f32() const { return !std::is_same<TX, double>::value && stage2_on() && st2.kind != VAL_F64; }
+
+    // Level 0's ends are taken over by the kernels around the V-cycle (Ends).
+    bool ends() const { return lv.size() > 1 && lv[0]->smoother == FS_COLOR_GS && lv[0]->dinv0.get(); }
+    const TX *end_dinv0() const { return ends() ? lv[0]->dinv0.get() : nullptr; }
+
+    // stage 1: L0.u = stage1_maxit AMG iterations on L0.f (the restriction has relaxed the first class), and z its
+    // prolongation
+    template <typename TZ>
+    void stage1(TZ *z, cudaStream_t s) {
         FastLevel<TX> &L0 = *lv[0];
-        constexpr bool fp64 = std::is_same<TX, double>::value;
-        const long long n = (long long)nb * bs;
-        if (fp64) {
-            launch_dep(fk::restrict_p<TX>, dim3(div_up(nb, kThreads)), dim3(kThreads), s,
-                       nb, bs, cfg.pressure_index, r, L0.f.get());
-        } else {
-            launch_dep(fk::restrict_cvt<TX>, dim3(div_up(n, kThreads)), dim3(kThreads), s,
-                       nb, bs, cfg.pressure_index, r, L0.f.get(),
-                                                                        r32.get());
-        }
-        JX_LAUNCH_CHECK();
-        vcycle_tx(L0.f.get(), L0.u.get(), s);
+        Ends E;
+        E.first_done = ends();
+        const bool fused = ends() && cfg.stage1_maxit <= 1;
+        if constexpr (std::is_same<TZ, double>::value) E.z64 = fused ? z : nullptr;
+        else E.z32 = fused ? z : nullptr;
+        vcycle_tx(L0.f.get(), L0.u.get(), s, E);
         for (int it = 1; it < cfg.stage1_maxit; ++it) {
             // further AMG iterations as residual corrections: u += V(f - A u)
             residual(L0, L0.f.get(), L0.u.get(), L0.r.get(), s);
@@ -1131,25 +1205,57 @@ struct FastCpr final : FastCprBase {
                        L0.c.get());
             JX_LAUNCH_CHECK();
         }
-        const bool st2_on = cfg.stage2_solver_type == 2 && cfg.stage2_maxit > 0;
-        if (fp64 || !st2_on || st2.kind == VAL_F64) {
-            // FP64 stage 2 on the caller's vectors (FP64 path; hybrid form: FP32 stage 1, FP64 polish)
-            launch_dep(fk::prolong_p<TX, double>, dim3(div_up(n, kThreads)), dim3(kThreads), s,
-                       nb, bs, cfg.pressure_index,
-                                                                              L0.u.get(), z);
+        if (fused) return;
+        const long long n = (long long)nb * bs;
+        launch_dep(fk::prolong_p<TX, TZ>, dim3(div_up(n, kThreads)), dim3(kThreads), s, nb, bs, cfg.pressure_index,
+                   L0.u.get(), z);
+        JX_LAUNCH_CHECK();
+    }
+    // native_f32: both stages from L0.f and r32 to z32
+    void stages_f32(cudaStream_t s) {
+        stage1(z32.get(), s);
+        for (int it = 0; it < cfg.stage2_maxit; ++it) sweep_typed<float>(r32.get(), z32.get(), vt32.get(), s);
+    }
+    // L0.f and r32 (mixed path) from r, or from basis vector V[*i]
+    template <typename TB>
+    void restrict_to(const TB *r, const TB *const *V, const int *i, cudaStream_t s) {
+        FastLevel<TX> &L0 = *lv[0];
+        if constexpr (std::is_same<TX, double>::value) {
+            launch_dep(fk::restrict_p<TX>, dim3(div_up(nb, kThreads)), dim3(kThreads), s, nb, bs, cfg.pressure_index,
+                       r, L0.f.get(), end_dinv0(), L0.u.get());
+        } else {
+            launch_dep(fk::restrict_cvt<TX, TB>, dim3(div_up((long long)nb * bs, kThreads)), dim3(kThreads), s, nb, bs,
+                       cfg.pressure_index, r, V, i, L0.f.get(), r32.get(), end_dinv0(), L0.u.get());
+        }
+        JX_LAUNCH_CHECK();
+    }
+
+    void apply_direct(const double *r, double *z, cudaStream_t s) {
+        DepLaunchScope dep(opt.dep_launch);
+        const long long n = (long long)nb * bs;
+        restrict_to<double>(r, nullptr, nullptr, s);
+        if (native_f32()) {
+            stages_f32(s);
+            launch_dep(fk::convert<float, double>, dim3(div_up(n, kThreads)), dim3(kThreads), s, n, z32.get(), z);
             JX_LAUNCH_CHECK();
-            if (st2_on)
-                for (int it = 0; it < cfg.stage2_maxit; ++it) sweep_typed<double>(r, z, vt.get(), s);
             return;
         }
-        // mixed path: stage 2 on FP32 copies of r and z, result converted to FP64
-        launch_dep(fk::prolong_p<TX, float>, dim3(div_up(n, kThreads)), dim3(kThreads), s,
-                   nb, bs, cfg.pressure_index, L0.u.get(),
-                                                                         z32.get());
-        JX_LAUNCH_CHECK();
-        for (int it = 0; it < cfg.stage2_maxit; ++it) sweep_typed<float>(r32.get(), z32.get(), vt32.get(), s);
-        launch_dep(fk::convert<float, double>, dim3(div_up(n, kThreads)), dim3(kThreads), s, n, z32.get(), z);
-        JX_LAUNCH_CHECK();
+        // FP64 stage 2 on the caller's vectors (FP64 path; hybrid form: FP32 stage 1, FP64 polish)
+        stage1(z, s);
+        if (stage2_on())
+            for (int it = 0; it < cfg.stage2_maxit; ++it) sweep_typed<double>(r, z, vt.get(), s);
+    }
+
+    const float *apply_enqueue_basis(const float *const *v32, const double *const *v64, const int *i,
+                                     cudaStream_t s) override {
+        if (!native_f32()) return nullptr;
+        if constexpr (!std::is_same<TX, double>::value) {
+            DepLaunchScope dep(opt.dep_launch);
+            if (v32) restrict_to<float>(nullptr, v32, i, s);
+            else restrict_to<double>(nullptr, v64, i, s);
+            stages_f32(s);
+        }
+        return z32.get();
     }
 
     void vcycle(const double *fp, double *up, cudaStream_t s) override {
@@ -1357,13 +1463,68 @@ static FastCprBase *build_fast(Amg &H, const BsrView<double> &A, const CprConfig
                 alloc_vec(Lv.y2, n);
                 H.log.mark("fast_lambda_max", s);
             }
+            if (l == 0 && sm == FS_COLOR_GS) {
+                alloc_vec(Lv.dinv0, n);
+                Lv.dinv0.zero(s);
+                if (n) {
+                    fk::dinv_class0<TX><<<div_up(n, kThreads), kThreads, 0, s>>>(
+                        HL.fwd.h_group_ptr[1], HL.fwd.perm.get(), Lv.dinv.get(), Lv.dinv0.get());
+                    JX_LAUNCH_CHECK();
+                }
+            }
             alloc_vec(Lv.r, n);
+            Lv.r.zero(s);  // entries no residual writes (class 0 of level 0) meet R's padding: finite
             alloc_vec(Lv.z, n);
             if (l == 0) alloc_vec(Lv.c, n);
             const int pk = fp64 ? VAL_F64 : VAL_F32;  // transfer operators: FP32 in the mixed path
-            const CsrView<double> Pv = HL.P.view(), Rv = HL.R.view();
-            build_tuned<TX>(("P" + std::to_string(l)).c_str(), Pv.nrows, Pv.ncols, Pv.nnz, Pv.ia, Pv.ja, Pv.a, pk, {},
-                            {}, nullptr, opt, Lv.P, F->tune_log, s);
+            const CsrView<double> Pv = HL.P.view();
+            CsrView<double> Rv = HL.R.view();
+            DeviceCsr Rkept;
+            if (l == 0 && sm == FS_COLOR_GS && Lv.smoother_plain == FS_COLOR_GS && n > 0) {
+                DevBuf<unsigned char> skip(n);
+                DevBuf<int> zeros(1);
+                zeros.zero(s);
+                fk::class0_flags<TX><<<div_up(n, kThreads), kThreads, 0, s>>>(
+                    n, HL.fwd.h_group_ptr[1], HL.fwd.perm.get(), Lv.dinv.get(), skip.get(), zeros.get());
+                JX_LAUNCH_CHECK();
+                int nz = 0;
+                zeros.download(&nz, 1, s);
+                JX_CUDA(cudaStreamSynchronize(s));
+                if (nz == 0) {
+                    Lv.skip_class0 = true;
+                    DevBuf<int> len(Rv.nrows + 1);
+                    len.zero(s);
+                    Rkept.nrows = Rv.nrows;
+                    Rkept.ncols = Rv.ncols;
+                    Rkept.ia.alloc((size_t)Rv.nrows + 1);
+                    int knnz = 0;
+                    if (Rv.nrows > 0) {
+                        fk::kept_len<<<div_up(Rv.nrows, kThreads), kThreads, 0, s>>>(Rv.nrows, Rv.ia, Rv.ja,
+                                                                                    skip.get(), len.get());
+                        JX_LAUNCH_CHECK();
+                    }
+                    exclusive_scan_int(len.get(), Rkept.ia.get(), Rv.nrows + 1, s);
+                    JX_CUDA(cudaMemcpyAsync(&knnz, Rkept.ia.get() + Rv.nrows, sizeof(int), cudaMemcpyDeviceToHost, s));
+                    JX_CUDA(cudaStreamSynchronize(s));
+                    Rkept.nnz = knnz;
+                    Rkept.ja.alloc(knnz > 0 ? knnz : 1);
+                    Rkept.a.alloc(knnz > 0 ? knnz : 1);
+                    if (Rv.nrows > 0) {
+                        fk::kept_copy<<<div_up(Rv.nrows, kThreads), kThreads, 0, s>>>(
+                            Rv.nrows, Rv.ia, Rv.ja, Rv.a, skip.get(), Rkept.ia.get(), Rkept.ja.get(), Rkept.a.get());
+                        JX_LAUNCH_CHECK();
+                    }
+                    Rv = Rkept.view();
+                }
+            }
+            if (Lv.skip_class0) {
+                std::vector<int> order = download_ints(HL.fwd.perm.get(), n, s);
+                build_tuned<TX>("P0", Pv.nrows, Pv.ncols, Pv.nnz, Pv.ia, Pv.ja, Pv.a, pk, order,
+                                {0, HL.fwd.h_group_ptr[1], n}, HL.fwd.perm.get(), opt, Lv.P, F->tune_log, s);
+            } else {
+                build_tuned<TX>(("P" + std::to_string(l)).c_str(), Pv.nrows, Pv.ncols, Pv.nnz, Pv.ia, Pv.ja, Pv.a, pk,
+                                {}, {}, nullptr, opt, Lv.P, F->tune_log, s);
+            }
             build_tuned<TX>(("R" + std::to_string(l)).c_str(), Rv.nrows, Rv.ncols, Rv.nnz, Rv.ia, Rv.ja, Rv.a, pk, {},
                             {}, nullptr, opt, Lv.R, F->tune_log, s);
             H.log.mark("fast_transfers", s);

@@ -33,27 +33,15 @@ __device__ __forceinline__ TA group_sum(TA v) {
     return v;
 }
 
-// sum_{k in [kb, ke)} a_k x_{ja_k}, reduced over the V lanes of the group.
-// Two entries per lane per trip keep more loads in flight; each product is added with one fused
-// multiply-add (the fast path has no bit-exactness contract; the exact path's kernels do not use it).
-template <int V, typename TA, typename TV, typename TX>
-__device__ __forceinline__ TA row_sum(const int *__restrict__ ja, const TV *__restrict__ a, const float *bsc, int kb,
-                                      int ke, const TX *x, int lane) {
-    TA s0 = 0, s1 = 0;
-    int k = kb + lane;
-    for (; k + V < ke; k += 2 * V) {
-        const int j0 = __ldg(ja + k), j1 = __ldg(ja + k + V);
-        const TA a0 = (TA)ldvs(a, bsc, k), a1 = (TA)ldvs(a, bsc, k + V);
-        s0 = fma(a0, (TA)x[j0], s0);
-        s1 = fma(a1, (TA)x[j1], s1);
-    }
-    if (k < ke) s0 = fma((TA)ldvs(a, bsc, k), (TA)x[__ldg(ja + k)], s0);
-    return group_sum<V, TA>(s0 + s1);
-}
-
 // ---- matrix formats -----------------------------------------------------------
-// CSR with V lanes per row.  Stored row t maps to vector row perm[t] (perm ==
-// nullptr: identity); bscale (BF16 storage): one scale per 32 consecutive stored values.
+// A format's row sum comes in two parts: head() reads the row's extent and its first entries, which
+// no kernel of a V-cycle writes, so it may run before the kernel ahead has finished; tail() gathers x.
+//
+// CSR with V lanes per row: sum_{k in [kb, ke)} a_k x_{ja_k}, reduced over the V lanes of the group.
+// Stored row t maps to vector row perm[t] (perm == nullptr: identity); bscale (BF16 storage): one
+// scale per 32 consecutive stored values.  Two entries per lane per trip keep more loads in flight;
+// each product is added with one fused multiply-add (the fast path has no bit-exactness contract; the
+// exact path's kernels do not use it).
 template <int V_, typename TV>
 struct CsrFmt {
     static constexpr int V = V_;
@@ -61,72 +49,119 @@ struct CsrFmt {
     const TV *a;
     const float *bscale;
     const int *perm;
+    template <typename TA>
+    struct Head {
+        int k, e;  // this lane's first entry, the row's end
+        int j0, j1;
+        TA a0, a1;
+    };
     __device__ __forceinline__ int row(int t) const { return perm ? __ldg(perm + t) : t; }
-    template <typename TA, typename TX>
-    __device__ __forceinline__ TA sum(int t, bool live, int lane, const TX *x, int kstart) const {
-        const int e = live ? __ldg(ia + t + 1) : 0;
+    template <typename TA>
+    __device__ __forceinline__ void head(int t, bool live, int lane, int kstart, Head<TA> &h) const {
+        h.e = live ? __ldg(ia + t + 1) : 0;
         int d = live ? __ldg(ia + t) + kstart : 0;
-        if (d > e) d = e;
-        return row_sum<V, TA>(ja, a, bscale, d, e, x, lane);
+        if (d > h.e) d = h.e;
+        h.k = d + lane;
+        h.j0 = h.j1 = 0;
+        h.a0 = h.a1 = 0;
+        if (h.k < h.e) {
+            h.j0 = __ldg(ja + h.k);
+            h.a0 = (TA)ldvs(a, bscale, h.k);
+        }
+        if (h.k + V < h.e) {
+            h.j1 = __ldg(ja + h.k + V);
+            h.a1 = (TA)ldvs(a, bscale, h.k + V);
+        }
+    }
+    template <typename TA, typename TX>
+    __device__ __forceinline__ TA tail(Head<TA> &h, const TX *x) const {
+        TA s0 = 0, s1 = 0;
+        if (h.k < h.e) s0 = h.a0 * (TA)x[h.j0];
+        if (h.k + V < h.e) s1 = h.a1 * (TA)x[h.j1];
+        int k = h.k + 2 * V;
+        for (; k + V < h.e; k += 2 * V) {
+            const int j0 = __ldg(ja + k), j1 = __ldg(ja + k + V);
+            const TA a0 = (TA)ldvs(a, bscale, k), a1 = (TA)ldvs(a, bscale, k + V);
+            s0 = fma(a0, (TA)x[j0], s0);
+            s1 = fma(a1, (TA)x[j1], s1);
+        }
+        if (k < h.e) s0 = fma((TA)ldvs(a, bscale, k), (TA)x[__ldg(ja + k)], s0);
+        return group_sum<V, TA>(s0 + s1);
     }
 };
 
-// Sliced ELL: 32-row slices stored slot-major, entry k of stored row t at
-// sp[t/32] + 32 k + t%32 (padding: value 0, column 0).  rows[t] is the vector
-// row of stored row t (-1: padding row).  One thread per row: the 32 rows of a
-// warp read each slot with one coalesced access.
-// P = 2: two lanes per row.  Stored row t is split into the virtual rows 2t and 2t + 1, holding its
-// entries of even and odd position; the virtual rows form the 32-row slices (16 stored rows each),
-// and the pair's sums are added with one shuffle.
+// Sliced ELL with P lanes per row (P = 1 .. 32, a power of two).  Stored row t is split into the virtual
+// rows P t + h, h < P, holding its entries of positions h, h + P, ...; slices of 32 virtual rows are
+// stored slot-major, entry k of virtual row v at sp[v/32] + 32 k + v%32 (padding: value 0, column 0), so
+// a warp reads each slot of its 32 virtual rows with one coalesced access and the P sums of a row are
+// added with shuffles.  rows[t] is the vector row of stored row t (-1: padding row).  Slots are read in
+// batches of NB, a batch ahead of the gathers it feeds; a slice's width is the same for the whole warp,
+// so the batch's last slots are skipped without divergence.
 template <typename TV, int P = 1>
 struct SellFmt {
     static constexpr int V = P;
+    static constexpr int NB = sizeof(TV) == 8 ? 4 : 8;  // slots per batch
     const long long *sp;
     const int *col;
     const TV *a;
-    const float *bscale;  // BF16: one scale per 32 stored values (one slot of a slice)
+    const float *bscale;  // BF16 (P = 1): one scale per 32 stored values (one slot of a slice)
     const int *rows;
+    template <typename TA>
+    struct Head {
+        long long o;  // slot 0 of the virtual row
+        int k, w;     // first slot of the sum, the slice's width
+        int j[NB];
+        TA a[NB];
+    };
     __device__ __forceinline__ int row(int t) const { return __ldg(rows + t); }
-    template <typename TA, typename TX>
-    __device__ __forceinline__ TA sum(int t, bool live, int lane, const TX *x, int kstart) const {
-        if constexpr (P == 1) {
-            if (!live) return 0;
-            return slots<TA>((long long)t, x, kstart);
-        } else {
-            // every lane takes part in the shuffle, live or not; lane h holds positions h, h + P, ...
-            const TA s = live ? slots<TA>((long long)t * P + lane, x, kstart > lane ? (kstart - lane + P - 1) / P : 0)
-                              : (TA)0;
-            return group_sum<P, TA>(s);
-        }
+    template <typename TA>
+    __device__ __forceinline__ void batch(long long o, int k, int w, int (&j)[NB], TA (&v)[NB]) const {
+        const long long p = o + (long long)k * 32;
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+            if (k + q < w) {
+                j[q] = __ldg(col + p + 32 * q);
+                v[q] = (TA)ldvs(a, bscale, p + 32 * q);
+            }
     }
-    // slots [kstart, width) of virtual row vt
+    template <typename TA>
+    __device__ __forceinline__ void head(int t, bool live, int lane, int kstart, Head<TA> &h) const {
+        const long long vt = (long long)t * P + lane;
+        h.k = kstart > lane ? (kstart - lane + P - 1) / P : 0;  // first position >= kstart
+        h.o = 0;
+        h.w = 0;
+        if (live) {
+            const long long b0 = __ldg(sp + (vt >> 5)), b1 = __ldg(sp + (vt >> 5) + 1);
+            h.w = (int)((b1 - b0) >> 5);
+            h.o = b0 + (vt & 31);
+        }
+        batch(h.o, h.k, h.w, h.j, h.a);
+    }
     template <typename TA, typename TX>
-    __device__ __forceinline__ TA slots(long long vt, const TX *x, int kstart) const {
-        const long long b0 = __ldg(sp + (vt >> 5)), b1 = __ldg(sp + (vt >> 5) + 1);
-        const int w = (int)((b1 - b0) >> 5);
-        const long long o = b0 + (vt & 31);
-        TA s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-        int k = kstart;
-        for (; k + 3 < w; k += 4) {
-            const long long p = o + (long long)k * 32;
-            const int j0 = __ldg(col + p), j1 = __ldg(col + p + 32), j2 = __ldg(col + p + 64),
-                      j3 = __ldg(col + p + 96);
-            const TA a0 = (TA)ldvs(a, bscale, p), a1 = (TA)ldvs(a, bscale, p + 32), a2 = (TA)ldvs(a, bscale, p + 64),
-                     a3 = (TA)ldvs(a, bscale, p + 96);
-            s0 = fma(a0, (TA)x[j0], s0);
-            s1 = fma(a1, (TA)x[j1], s1);
-            s2 = fma(a2, (TA)x[j2], s2);
-            s3 = fma(a3, (TA)x[j3], s3);
+    __device__ __forceinline__ TA tail(Head<TA> &h, const TX *x) const {
+        TA s[4] = {0, 0, 0, 0};
+        const int w = h.w;
+        for (int k = h.k; k < w; k += NB) {
+            TA xv[NB];
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+                if (k + q < w) xv[q] = (TA)x[h.j[q]];
+            TA av[NB];
+#pragma unroll
+            for (int q = 0; q < NB; ++q) av[q] = h.a[q];
+            batch(h.o, k + NB, w, h.j, h.a);
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+                if (k + q < w) s[q & 3] = fma(av[q], xv[q], s[q & 3]);
         }
-        for (; k < w; ++k) {
-            const long long p = o + (long long)k * 32;
-            s0 = fma((TA)ldvs(a, bscale, p), (TA)x[__ldg(col + p)], s0);
-        }
-        return (s0 + s1) + (s2 + s3);
+        // every lane takes part in the row's shuffles, live or not
+        return group_sum<P, TA>((s[0] + s[1]) + (s[2] + s[3]));
     }
 };
 
-// ---- row operations (prologue loads issued before the row sum) -----------------
+// ---- row operations ------------------------------------------------------------
+// early(): the row's constants, read before the kernel ahead has finished; load(): its vector entries,
+// issued before the row sum; store(): the result.
 // Gauss-Seidel on one colour class: u_i = (f_i - sum_{j != i} a_ij u_j) dinv_i
 // (the diagonal is the first stored entry; dinv_i == 0 leaves the row).
 template <typename TX>
@@ -134,13 +169,26 @@ struct OpGs {
     static constexpr int kstart = 1;
     const TX *f, *dinv;
     TX *u;
-    int zero;  // every neighbour is 0 (first class after u = 0)
     struct Pre { TX f, d; };
     __device__ __forceinline__ const TX *x() const { return u; }
-    __device__ __forceinline__ bool need_sum() const { return !zero; }
-    __device__ __forceinline__ void load(int i, Pre &p) const { p.f = f[i]; p.d = dinv[i]; }
+    __host__ __device__ __forceinline__ bool need_sum() const { return true; }
+    __device__ __forceinline__ void early(int i, Pre &p) const { p.d = __ldg(dinv + i); }
+    __device__ __forceinline__ void load(int i, Pre &p) const { p.f = f[i]; }
     __device__ __forceinline__ void store(int i, TX s, const Pre &p) const {
         if (p.d != (TX)0) u[i] = (p.f - s) * p.d;
+    }
+};
+// The same where the class is relaxed for the last time in an application: the value also goes to component
+// p of cell i of z, the cell's other components are set to 0 (the prolongation of the pressure).
+template <typename TX, typename TZ>
+struct OpGsZ : OpGs<TX> {
+    TZ *z;
+    int bs, p;
+    using Pre = typename OpGs<TX>::Pre;
+    __device__ __forceinline__ void store(int i, TX s, const Pre &q) const {
+        const TX v = q.d != (TX)0 ? (q.f - s) * q.d : this->u[i];
+        this->u[i] = v;
+        for (int k = 0; k < bs; ++k) z[(long long)i * bs + k] = k == p ? (TZ)v : (TZ)0;
     }
 };
 // unew_i = u_i + (f_i - (A u)_i) dinv_i
@@ -152,10 +200,10 @@ struct OpJacobi {
     int zero;  // u == 0
     struct Pre { TX f, d, u; };
     __device__ __forceinline__ const TX *x() const { return u; }
-    __device__ __forceinline__ bool need_sum() const { return !zero; }
+    __host__ __device__ __forceinline__ bool need_sum() const { return !zero; }
+    __device__ __forceinline__ void early(int i, Pre &p) const { p.d = __ldg(dinv + i); }
     __device__ __forceinline__ void load(int i, Pre &p) const {
         p.f = f[i];
-        p.d = dinv[i];
         p.u = zero ? (TX)0 : u[i];
     }
     __device__ __forceinline__ void store(int i, TX s, const Pre &p) const { unew[i] = p.u + (p.f - s) * p.d; }
@@ -168,7 +216,8 @@ struct OpResid {
     TX *r;
     struct Pre { TX f; };
     __device__ __forceinline__ const TX *x() const { return u; }
-    __device__ __forceinline__ bool need_sum() const { return true; }
+    __host__ __device__ __forceinline__ bool need_sum() const { return true; }
+    __device__ __forceinline__ void early(int, Pre &) const {}
     __device__ __forceinline__ void load(int i, Pre &p) const { p.f = f[i]; }
     __device__ __forceinline__ void store(int i, TX s, const Pre &p) const { r[i] = p.f - s; }
 };
@@ -181,9 +230,30 @@ struct OpSpmv {
     int beta_one;
     struct Pre { TX y; };
     __device__ __forceinline__ const TX *x() const { return xin; }
-    __device__ __forceinline__ bool need_sum() const { return true; }
+    __host__ __device__ __forceinline__ bool need_sum() const { return true; }
+    __device__ __forceinline__ void early(int, Pre &) const {}
     __device__ __forceinline__ void load(int i, Pre &p) const { p.y = beta_one ? y[i] : (TX)0; }
     __device__ __forceinline__ void store(int i, TX s, const Pre &p) const { y[i] = beta_one ? p.y + s : s; }
+};
+// f = R r, and on the coarse level the first step of its smoother from a zero iterate, which needs no
+// neighbours: z = D^-1 f (l1-Jacobi's first iterate), y = c z (the polynomial's first step; nullptr: none).
+template <typename TX>
+struct OpRestrict {
+    static constexpr int kstart = 0;
+    const TX *xin, *dinv;
+    TX *f, *z, *y;
+    TX c;
+    struct Pre { TX d; };
+    __device__ __forceinline__ const TX *x() const { return xin; }
+    __host__ __device__ __forceinline__ bool need_sum() const { return true; }
+    __device__ __forceinline__ void early(int i, Pre &p) const { p.d = __ldg(dinv + i); }
+    __device__ __forceinline__ void load(int, Pre &) const {}
+    __device__ __forceinline__ void store(int i, TX s, const Pre &p) const {
+        f[i] = s;
+        const TX zi = s * p.d;
+        z[i] = zi;
+        if (y) y[i] = c * zi;
+    }
 };
 // Degree-3 polynomial smoother, Horner form of u += p(M) z, M = D^-1 A,
 // z = D^-1 (f - A u), p(t) = c0 + c1 t + c2 t^2:
@@ -199,9 +269,9 @@ struct OpCheb {
     TX *u, *z, *yout;
     struct Pre { TX d, a, b; };
     __device__ __forceinline__ const TX *x() const { return mode == 0 ? u : yin; }
-    __device__ __forceinline__ bool need_sum() const { return !(mode == 0 && zero); }
+    __host__ __device__ __forceinline__ bool need_sum() const { return !(mode == 0 && zero); }
+    __device__ __forceinline__ void early(int i, Pre &p) const { p.d = __ldg(dinv + i); }
     __device__ __forceinline__ void load(int i, Pre &p) const {
-        p.d = dinv[i];
         if (mode == 0) {
             p.a = f[i];
         } else {
@@ -222,10 +292,11 @@ struct OpCheb {
     }
 };
 
-// One launch of `op` over stored rows [r0, r1) of a matrix in format Fmt.
+// One launch of `op` over stored rows [r0, r1) of a matrix in format Fmt.  The row's extent, first
+// entries and constants are read before the wait for the kernel ahead: on the coarse levels, whose
+// passes take a few microseconds, these reads were the first half of each pass's chain of latencies.
 template <class Fmt, class Op, typename TX>
 __global__ void __launch_bounds__(256) row_kernel(Fmt fmt, Op op, int r0, int r1) {
-    grid_dep_wait();
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int t = r0 + (int)(gt / Fmt::V);
     const int lane = (int)(gt % Fmt::V);
@@ -233,21 +304,59 @@ __global__ void __launch_bounds__(256) row_kernel(Fmt fmt, Op op, int r0, int r1
     const int i = live ? fmt.row(t) : -1;
     const bool own = i >= 0 && lane == 0;
     typename Op::Pre pre;
+    typename Fmt::template Head<TX> h;
+    if (op.need_sum()) fmt.template head<TX>(t, i >= 0, lane, Op::kstart, h);
+    if (own) op.early(i, pre);
+    grid_dep_wait();
     if (own) op.load(i, pre);
     TX s = 0;
-    if (op.need_sum()) s = fmt.template sum<TX, TX>(t, i >= 0, lane, op.x(), Op::kstart);
+    if (op.need_sum()) s = fmt.template tail<TX, TX>(h, op.x());
     if (own) op.store(i, s, pre);
 }
 
+// The first Gauss-Seidel colour class from a zero iterate, u_i = f_i dinv_i for the stored rows below
+// `cend`, and u = 0 on the other rows: one launch in place of a memset and a class pass (a memset
+// between the kernels of a V-cycle also keeps the next one from starting early).
+// rows: vector row of each stored row (-1: padding; nullptr: identity).
 template <typename TX>
-__global__ void restrict_p(int nb, int bs, int p, const double *__restrict__ r, TX *__restrict__ rp) {
+__global__ void gs_first_class(int nstored, int cend, const int *__restrict__ rows, const TX *f,
+                               const TX *__restrict__ dinv, TX *u) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t < nstored ? (rows ? __ldg(rows + t) : t) : -1;
+    const TX d = i >= 0 && t < cend ? __ldg(dinv + i) : (TX)0;
     grid_dep_wait();
+    if (i >= 0) u[i] = d != (TX)0 ? f[i] * d : (TX)0;
+}
+
+template <typename TX>
+__global__ void zero_rows(int nstored, const int *__restrict__ rows, TX *r) {
+    grid_dep_wait();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t < nstored ? (rows ? __ldg(rows + t) : t) : -1;
+    if (i >= 0) r[i] = (TX)0;
+}
+
+// The restriction also relaxes the first colour class from a zero iterate where level 0 is smoothed by
+// multicolour Gauss-Seidel: dinv0 (nullptr: not wanted) holds 1 / a_ii on class 0 and 0 elsewhere, and
+// u_i = f_i dinv0_i is what gs_first_class leaves.
+template <typename TX>
+__device__ __forceinline__ void first_class(const TX *dinv0, TX *u, int i, TX d, TX f) {
+    if (dinv0) u[i] = d != (TX)0 ? f * d : (TX)0;
+}
+
+template <typename TX>
+__global__ void restrict_p(int nb, int bs, int p, const double *r, TX *rp, const TX *__restrict__ dinv0, TX *u) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nb) rp[i] = (TX)r[(long long)i * bs + p];
+    const TX d = dinv0 && i < nb ? __ldg(dinv0 + i) : (TX)0;
+    grid_dep_wait();
+    if (i >= nb) return;
+    const TX f = (TX)r[(long long)i * bs + p];
+    rp[i] = f;
+    first_class(dinv0, u, i, d, f);
 }
 
 template <typename TX, typename TZ>
-__global__ void prolong_p(int nb, int bs, int p, const TX *__restrict__ up, TZ *__restrict__ z) {
+__global__ void prolong_p(int nb, int bs, int p, const TX *up, TZ *z) {
     grid_dep_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)nb * bs) return;
@@ -255,27 +364,54 @@ __global__ void prolong_p(int nb, int bs, int p, const TX *__restrict__ up, TZ *
     z[t] = k == p ? (TZ)up[i] : (TZ)0;
 }
 
-// rp = r[p-th component] and r32 = r converted (mixed path: stage 2 works in FP32)
-template <typename TX>
-__global__ void restrict_cvt(int nb, int bs, int p, const double *__restrict__ r, TX *__restrict__ rp,
-                             float *__restrict__ r32) {
-    grid_dep_wait();
+// rp = r[p-th component] and r32 = r converted (mixed path: stage 2 works in FP32), from r or (V != nullptr)
+// from vector V[*iv] of a Krylov basis.
+template <typename TX, typename TB>
+__global__ void restrict_cvt(int nb, int bs, int p, const TB *r, const TB *const *V, const int *iv, TX *rp, float *r32,
+                             const TX *__restrict__ dinv0, TX *u) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)nb * bs) return;
-    const double v = r[t];
+    const bool live = t < (long long)nb * bs;
+    const int i = live ? (int)(t / bs) : 0;
+    const bool mine = live && (int)(t % bs) == p;
+    const TX d = dinv0 && mine ? __ldg(dinv0 + i) : (TX)0;
+    grid_dep_wait();
+    if (!live) return;
+    const TB v = V ? V[*iv][t] : r[t];
     r32[t] = (float)v;
-    if ((int)(t % bs) == p) rp[t / bs] = (TX)v;
+    if (mine) {
+        rp[i] = (TX)v;
+        first_class(dinv0, u, i, d, (TX)v);
+    }
 }
 
-// u = Ainv f (FP64 inverse of the coarsest operator), one warp per row.
+// u = Ainv f (FP64 inverse of the coarsest operator), one warp per row; the row's first 256 entries
+// are read before the kernel ahead has finished, the rest eight loads per lane at a time.
 template <typename TX>
-__global__ void dense_gemv(int n, const double *__restrict__ Ainv, const TX *__restrict__ f, TX *__restrict__ u) {
-    grid_dep_wait();
+__global__ void dense_gemv(int n, const double *__restrict__ Ainv, const TX *f, TX *u) {
     const int row = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
+    const double *a = Ainv + (long long)row * n;
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int c = lane + 32 * q;
+        v[q] = row < n && c < n ? __ldg(a + c) : 0.0;
+    }
+    grid_dep_wait();
     if (row >= n) return;
     double s = 0.0;
-    for (int c = lane; c < n; c += 32) s += Ainv[(long long)row * n + c] * (double)f[c];
+    for (int c0 = lane; c0 < n; c0 += 256) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = c0 + 32 * q;
+            if (c < n) s += v[q] * (double)f[c];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = c0 + 256 + 32 * q;
+            v[q] = c < n ? __ldg(a + c) : 0.0;
+        }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) u[row] = (TX)s;
@@ -375,12 +511,12 @@ struct SweepOrder {
 template <typename TA, typename TXV>
 __device__ __forceinline__ TA start_value(const TXV *x, TXV *vt, long long o, int j, SweepOrder so) {
     const bool earlier = so.nmode == 1 || (so.nmode == 2 && __ldg(so.cls + j) < so.cur);
-    return earlier ? (TA)__ldg(vt + o) : (TA)x[o];
+    return earlier ? (TA)vt[o] : (TA)x[o];
 }
 
 template <int BS, int V, typename TV, typename TA, typename TXV>
 __global__ void hgs_color(int r0, int r1, const int *__restrict__ perm, const int *__restrict__ ia,
-                          const int *__restrict__ ja, const TV *__restrict__ a, const TXV *__restrict__ b,
+                          const int *__restrict__ ja, const TV *__restrict__ a, const TXV *b,
                           TXV *x, TXV *vt, TA w, TA omega, int plain, SweepOrder so) {
     grid_dep_wait();
     const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -430,7 +566,7 @@ __global__ void hgs_color(int r0, int r1, const int *__restrict__ perm, const in
 template <int BS, typename TV, typename TA, typename TXV>
 __global__ void __launch_bounds__(256) hgs_sell(int r0, int r1, const long long *__restrict__ sp,
                                                 const int *__restrict__ col, const TV *__restrict__ a,
-                                                const int *__restrict__ rows, const TXV *__restrict__ b,
+                                                const int *__restrict__ rows, const TXV *b,
                                                 TXV *x, TXV *vt, TA w, TA omega, int plain, SweepOrder so) {
     grid_dep_wait();
     const int t = r0 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -444,7 +580,7 @@ __global__ void __launch_bounds__(256) hgs_sell(int r0, int r1, const long long 
     TA rhs[BS], xv[BS], D[BS * BS], acc[BS];
 #pragma unroll
     for (int q = 0; q < BS; ++q) {
-        rhs[q] = (TA)__ldg(b + (long long)i * BS + q);
+        rhs[q] = (TA)b[(long long)i * BS + q];
         xv[q] = plain ? (TA)0 : (TA)x[(long long)i * BS + q];
         acc[q] = 0;
     }
@@ -542,17 +678,16 @@ __device__ __forceinline__ void block_matvec(const TA M[BS * BS], const TA v[BS]
 }
 
 // The two values of a 2-vector entry j of x (FP32: one 8-byte load; x's base is 8-byte aligned, which
-// the stage-2 launcher checks).  NC: through the read-only path, valid where no thread of the launch
-// writes the entry before it is read.
-template <typename TXV, typename TA, bool NC>
+// the stage-2 launcher checks).
+template <typename TXV, typename TA>
 __device__ __forceinline__ void ld_pair(const TXV *p, int j, TA out[2]) {
     if constexpr (sizeof(TXV) == 4) {
-        const float2 v = NC ? __ldg(reinterpret_cast<const float2 *>(p) + j) : reinterpret_cast<const float2 *>(p)[j];
+        const float2 v = reinterpret_cast<const float2 *>(p)[j];
         out[0] = (TA)v.x;
         out[1] = (TA)v.y;
     } else {
-        out[0] = (TA)(NC ? __ldg(p + 2LL * j) : p[2LL * j]);
-        out[1] = (TA)(NC ? __ldg(p + 2LL * j + 1) : p[2LL * j + 1]);
+        out[0] = (TA)p[2LL * j];
+        out[1] = (TA)p[2LL * j + 1];
     }
 }
 
@@ -567,15 +702,20 @@ constexpr unsigned kChunkColMask = 0x3fffffffu, kChunkEarlier = 1u << 30, kChunk
 // loaded after the entry loop, and for 2x2 blocks the kept in-chunk block is re-read by its slot
 // rather than held (measured on C1: 46.9 -> 41.1 us per sweep with the paired x gathers; C4: 103 ->
 // 79 us).
-template <int BS, int CH, typename TV, typename TA, typename TXV>
-__global__ void __launch_bounds__(256, sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) hgs_chunk(int r0, int r1, const long long *__restrict__ sp,
+// FEW: a colour of at most one block per SM, where nothing hides a row's chain of loads (a colour of 3
+// blocks took as long as one of 147).  The row keeps everything in registers: all six off-diagonal
+// entries of a 7-point row in one batch with the diagonal block, read before the wait; then every gather
+// at once with b and the row's own x, the start values through a selected address in place of a branch per
+// entry; the in-chunk block is held (145,297 2x2 rows in FP64, colours of 147 blocks: 9.9 -> 8.0 us,
+// of 3 blocks: 9.9 -> 7.0).
+template <int BS, int CH, typename TV, typename TA, typename TXV, bool FEW>
+__global__ void __launch_bounds__(256, FEW ? 1 : sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) hgs_chunk(int r0, int r1, const long long *__restrict__ sp,
                                                  const unsigned *__restrict__ col, const TV *__restrict__ a,
-                                                 const int *__restrict__ rows, const TXV *__restrict__ b,
+                                                 const int *__restrict__ rows, const TXV *b,
                                                  TXV *x, TXV *vt, TA w, TA omega, int plain, int save) {
     static_assert(32 % CH == 0, "chunks tile the 32-row slices");
-    constexpr bool kKeepSlot = BS == 2;  // hold the kept in-chunk block's slot, not its values
-    constexpr int NB = BS == 2 ? 4 : 2;  // entries loaded per batch
-    grid_dep_wait();
+    constexpr bool kKeepSlot = BS == 2 && !FEW;  // hold the kept in-chunk block's slot, not its values
+    constexpr int NB = FEW ? 6 : BS == 2 ? 4 : 2;  // entries loaded per batch
     const int t = r0 + blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int p = lane % CH;
@@ -592,10 +732,35 @@ __global__ void __launch_bounds__(256, sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) 
     for (int q = 0; q < BS * BS; ++q) G[q] = 0;
 #pragma unroll
     for (int q = 0; q < BS; ++q) u[q] = xv[q] = 0;
+    // the row's extent and its first batch of entries, read before the kernel ahead has finished
+    unsigned cw[NB];
+    TA B[NB][BS * BS], D[BS * BS], rhs[BS];
+    auto batch = [&](int k) {  // FEW: the slots below wd (the same for the whole warp)
+        const long long p0 = o + (long long)k * 32;
+#pragma unroll
+        for (int e = 0; e < NB; ++e)
+            if (!FEW || k + e < wd) {
+                cw[e] = __ldcs(col + p0 + 32 * e);
+                load_block_cs<BS, TV, TA>(a, p0 + 32 * e, B[e]);
+            }
+    };
+    auto own = [&]() {
+#pragma unroll
+        for (int q = 0; q < BS; ++q) {
+            rhs[q] = (TA)b[(long long)i * BS + q];
+            xv[q] = (TA)x[(long long)i * BS + q];
+        }
+    };
     if (live) {
         const long long b0 = __ldg(sp + (t >> 5)), b1 = __ldg(sp + (t >> 5) + 1);
         wd = (int)((b1 - b0) >> 5);
         o = b0 + (t & 31);
+        if (FEW) load_block_cs<BS, TV, TA>(a, o, D);
+        if (FEW || NB < wd) batch(1);
+    }
+    grid_dep_wait();
+    if (live) {
+        if (FEW) own();
         TA acc[BS], K[kKeepSlot ? 1 : BS * BS];
         int kslot = 0;  // slot of the kept in-chunk block (kKeepSlot)
 #pragma unroll
@@ -621,13 +786,11 @@ __global__ void __launch_bounds__(256, sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) 
                         kslot = kk;
                     }
                 }
-                // x is read-only within the launch where it is gathered: the chunks of one colour are
-                // not coupled, and the row's own chunk writes only after every lane's phase 1
                 TA xp[2], vp[2];
-                ld_pair<TXV, TA, true>(x, j, xp);
+                ld_pair<TXV, TA>(x, j, xp);
                 vp[0] = xp[0];
                 vp[1] = xp[1];
-                if (earlier_col) ld_pair<TXV, TA, true>(vt, j, vp);
+                if (earlier_col) ld_pair<TXV, TA>(vt, j, vp);
 #pragma unroll
                 for (int m = 0; m < BS; ++m) {
                     const TA base = same_earlier ? (TA)0 : xp[m];  // earlier in the chunk: -(1 - omega) A vt_j now
@@ -662,7 +825,7 @@ __global__ void __launch_bounds__(256, sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) 
                     for (int m = 0; m < BS; ++m) {
                         const long long oj = (long long)j * BS + m;
                         const TA xj = (TA)x[oj];
-                        c[m] = plain ? xj : xj - omo * (earlier ? (TA)__ldg(vt + oj) : xj);
+                        c[m] = plain ? xj : xj - omo * (earlier ? (TA)vt[oj] : xj);
                     }
                 }
             }
@@ -672,17 +835,53 @@ __global__ void __launch_bounds__(256, sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) 
                 for (int m = 0; m < BS; ++m) acc[q] += B[q * BS + m] * c[m];
         };
         int k = 1;
-        for (; k + NB - 1 < wd; k += NB) {
-            const long long p0 = o + (long long)k * 32;
-            unsigned cw[NB];
-            TA B[NB][BS * BS];
+        if constexpr (FEW) {
+            while (k < wd) {
+                TA xp[NB][BS], vp[NB][BS];
 #pragma unroll
-            for (int e = 0; e < NB; ++e) {
-                cw[e] = __ldcs(col + p0 + 32 * e);
-                load_block_cs<BS, TV, TA>(a, p0 + 32 * e, B[e]);
+                for (int e = 0; e < NB; ++e)
+                    if (k + e < wd) {
+                        const long long j = (long long)(cw[e] & kChunkColMask) * BS;
+                        const TXV *v = (cw[e] & kChunkEarlier) ? vt : x;
+#pragma unroll
+                        for (int m = 0; m < BS; ++m) {
+                            xp[e][m] = (TA)x[j + m];
+                            vp[e][m] = (TA)v[j + m];
+                        }
+                    }
+#pragma unroll
+                for (int e = 0; e < NB; ++e)
+                    if (k + e < wd) {
+                        const int dq = (int)(cw[e] & kChunkColMask) - cbase;
+                        const bool before = (cw[e] & kChunkSame) && dq <= p;  // an earlier row of the chunk
+                        if (before) {
+                            lowmask |= 1u << dq;
+                            if (kq < 0) {
+                                kq = dq;
+#pragma unroll
+                                for (int q = 0; q < BS * BS; ++q) K[q] = B[e][q];
+                            }
+                        }
+                        TA c[BS];
+#pragma unroll
+                        for (int m = 0; m < BS; ++m) {
+                            const TA base = before ? (TA)0 : xp[e][m];
+                            c[m] = plain ? base : base - omo * vp[e][m];
+                        }
+#pragma unroll
+                        for (int q = 0; q < BS; ++q)
+#pragma unroll
+                            for (int m = 0; m < BS; ++m) acc[q] += B[e][q * BS + m] * c[m];
+                    }
+                k += NB;
+                batch(k);
             }
+        }
+        while (k + NB - 1 < wd) {
 #pragma unroll
             for (int e = 0; e < NB; ++e) entry(cw[e], B[e], k + e);
+            k += NB;
+            if (k + NB - 1 < wd) batch(k);
         }
         for (; k < wd; ++k) {
             const long long p0 = o + (long long)k * 32;
@@ -690,13 +889,10 @@ __global__ void __launch_bounds__(256, sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) 
             load_block_cs<BS, TV, TA>(a, p0, B0);
             entry(__ldcs(col + p0), B0, k);
         }
-        TA rhs[BS], D[BS * BS];
-#pragma unroll
-        for (int q = 0; q < BS; ++q) {
-            rhs[q] = (TA)__ldg(b + (long long)i * BS + q);
-            xv[q] = (TA)x[(long long)i * BS + q];
+        if (!FEW) {
+            own();
+            load_block_cs<BS, TV, TA>(a, o, D);
         }
-        load_block_cs<BS, TV, TA>(a, o, D);
         block_inverse<BS, TA>(D, Di);
         TA r2[BS];
 #pragma unroll
@@ -872,35 +1068,34 @@ __global__ void sell_fill(int nstored, const int *__restrict__ rows, const long 
 }
 
 // The sliced ELL with P lanes per stored row (SellFmt<TV, P>, P > 1; FP32 / FP64 values, no block
-// scales): thread u is virtual row u (stored row u / P, lane u % P); the entry at (sorted) position
-// q of the row goes to lane q % P, slot q / P.  Unfilled slots are padding (value 0, column 0).
+// scales), a warp per stored row: the entry at (sorted) position q of the row goes to virtual row
+// P t + q % P, slot q / P.  Unfilled slots are padding (value 0, column 0).
 template <typename TV>
 __global__ void sell_fill_lanes(int nstored, int P, const int *__restrict__ rows, const long long *__restrict__ sp,
                                 const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ a,
                                 int *__restrict__ col, TV *__restrict__ val, int sorted) {
-    const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= (long long)nstored * P) return;
-    const int t = (int)(u / P), h = (int)(u % P);
+    const int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (t >= nstored) return;
     const int i = rows[t];
-    const long long b0 = sp[u >> 5], b1 = sp[(u >> 5) + 1];
-    const int w = (int)((b1 - b0) >> 5);
-    const long long o = b0 + (u & 31);
     const int d = i >= 0 ? ia[i] : 0, len = i >= 0 ? ia[i + 1] - d : 0;
-    for (int k = 0; k < w; ++k)
-        if (h + (long long)P * k >= len) {
-            col[o + (long long)k * 32] = 0;
-            val[o + (long long)k * 32] = cvt_val<TV>(0.0, 1.0);
-        }
-    for (int e = 0; e < len; ++e) {
+    // the P virtual rows lie in one slice (P divides 32)
+    const long long v0 = (long long)t * P, b0 = sp[v0 >> 5], b1 = sp[(v0 >> 5) + 1];
+    const int w = (int)((b1 - b0) >> 5);
+    const long long o = b0 + (v0 & 31);
+    for (int q = len + lane; q < w * P; q += 32) {
+        const long long pp = o + q % P + 32LL * (q / P);
+        col[pp] = 0;
+        val[pp] = cvt_val<TV>(0.0, 1.0);
+    }
+    for (int e = lane; e < len; e += 32) {
+        const int je = ja[d + e];
         int q = e;
         if (sorted && e > 0) {
-            const int je = ja[d + e];
             q = 1;
             for (int f = 1; f < len; ++f) q += ja[d + f] < je || (ja[d + f] == je && f < e);
         }
-        if (q % P != h) continue;
-        const long long pp = o + (long long)(q / P) * 32;
-        col[pp] = ja[d + e];
+        const long long pp = o + q % P + 32LL * (q / P);
+        col[pp] = je;
         val[pp] = cvt_val<TV>(a[d + e], 1.0);
     }
 }
@@ -945,6 +1140,44 @@ __global__ void to_bf16_blocks(long long nnz, const double *__restrict__ a, floa
     if (k < nnz) out[k] = __float2bfloat16_rn((float)(v / sc));
 }
 
+// dinv0 = dinv on the rows perm[0 .. cend)
+template <typename TX>
+__global__ void dinv_class0(int cend, const int *__restrict__ perm, const TX *__restrict__ dinv, TX *__restrict__ dinv0) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < cend) dinv0[perm[t]] = dinv[perm[t]];
+}
+// skip[i] = 1 for the rows perm[0 .. cend); *zeros counts those with dinv 0 (rows the smoother leaves)
+template <typename TX>
+__global__ void class0_flags(int n, int cend, const int *__restrict__ perm, const TX *__restrict__ dinv,
+                             unsigned char *__restrict__ skip, int *__restrict__ zeros) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int i = perm[t];
+    skip[i] = t < cend;
+    if (t < cend && dinv[i] == (TX)0) atomicAdd(zeros, 1);
+}
+// rows without the entries in flagged columns: their lengths, then the entries
+__global__ void kept_len(int n, const int *__restrict__ ia, const int *__restrict__ ja,
+                         const unsigned char *__restrict__ skip, int *__restrict__ len) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int c = 0;
+    for (int k = ia[i]; k < ia[i + 1]; ++k) c += skip[ja[k]] ? 0 : 1;
+    len[i] = c;
+}
+__global__ void kept_copy(int n, const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ a,
+                          const unsigned char *__restrict__ skip, const int *__restrict__ oia, int *__restrict__ oja,
+                          double *__restrict__ oa) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int o = oia[i];
+    for (int k = ia[i]; k < ia[i + 1]; ++k)
+        if (!skip[ja[k]]) {
+            oja[o] = ja[k];
+            oa[o++] = a[k];
+        }
+}
+
 // 1 / a_ii where the diagonal is the first stored entry, else 0 (row skipped).
 template <typename TX>
 __global__ void dinv_diag(int n, const int *__restrict__ ia, const int *__restrict__ ja,
@@ -965,18 +1198,71 @@ __global__ void dinv_l1(int n, const int *__restrict__ ia, const double *__restr
     out[i] = s > 0.0 ? (TX)(1.0 / s) : (TX)0;
 }
 
-// y = D^-1 A x in FP64 (power iteration); dinv from dinv_diag<double>.
-__global__ void dinv_a_x(int n, const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ a,
-                         const double *__restrict__ dinv, const double *__restrict__ x, double *__restrict__ y) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = 0.0;
-    for (int k = ia[i]; k < ia[i + 1]; ++k) s += a[k] * x[ja[k]];
-    y[i] = dinv[i] * s;
+// One power step in FP64, V lanes per row: y = D^-1 A (c x) with c = st[1], and per block the partial sums of
+// <y, y> and <c x, c x> (part[block], part[gridDim.x + block]).  dinv from dinv_diag<double>.
+constexpr int kPowerThreads = 256;
+template <int V>
+__global__ void __launch_bounds__(kPowerThreads) power_step(int n, const int *__restrict__ ia,
+                                                            const int *__restrict__ ja, const double *__restrict__ a,
+                                                            const double *__restrict__ dinv, const double *x,
+                                                            const double *st, double *y, double *part) {
+    __shared__ double sh[2][kPowerThreads / 32];
+    const int lane = threadIdx.x % V, rows = gridDim.x * (kPowerThreads / V);
+    const double c = st[1];
+    double yy = 0.0, xx = 0.0;
+    const int per = (n + rows - 1) / rows;  // a uniform trip count: every lane reaches the shuffles
+    for (int t = 0; t < per; ++t) {
+        const int i = t * rows + (blockIdx.x * kPowerThreads + threadIdx.x) / V;
+        double s = 0.0;
+        if (i < n)
+            for (int k = ia[i] + lane; k < ia[i + 1]; k += V) s += a[k] * (c * x[ja[k]]);
+        s = group_sum<V, double>(s);
+        if (i < n && lane == 0) {
+            const double v = dinv[i] * s, xi = c * x[i];
+            y[i] = v;
+            yy += v * v;
+            xx += xi * xi;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        yy += __shfl_xor_sync(0xffffffffu, yy, o);
+        xx += __shfl_xor_sync(0xffffffffu, xx, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = yy;
+        sh[1][threadIdx.x >> 5] = xx;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double s = 0.0;
+        for (int q = 0; q < kPowerThreads / 32; ++q) s += sh[threadIdx.x][q];
+        part[threadIdx.x * gridDim.x + blockIdx.x] = s;
+    }
+}
+
+// The step's scalars: lam = sqrt(<y,y> / <x,x>) and the next iterate's factor 1 / ||y||, or the stop flag once
+// a norm is not positive (lam keeps its last value).  st = {lam, factor, stop}.
+__global__ void __launch_bounds__(64) power_scalars(int nblocks, const double *__restrict__ part, double *st) {
+    __shared__ double sum[2];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v = 0.0;
+    for (int i = lane; i < nblocks; i += 32) v += part[w * nblocks + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) sum[w] = v;
+    __syncthreads();
+    if (threadIdx.x != 0 || st[2] != 0.0) return;
+    if (!(sum[0] > 0.0) || !(sum[1] > 0.0)) {
+        st[2] = 1.0;
+        return;
+    }
+    st[0] = sqrt(sum[0] / sum[1]);
+    st[1] = 1.0 / sqrt(sum[0]);
 }
 
 template <typename TA, typename TB>
-__global__ void convert(long long n, const TA *__restrict__ in, TB *__restrict__ out) {
+__global__ void convert(long long n, const TA *in, TB *out) {
     grid_dep_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = (TB)in[i];

@@ -10,6 +10,8 @@
 // (the solve then reports a device error) and the kernel returns.
 #pragma once
 
+#include <type_traits>
+
 #include "fast.cuh"
 #include "fast_kernels.cuh"
 #include "grid_sync.cuh"
@@ -67,9 +69,16 @@ __device__ __forceinline__ void rows_pass(const Fmt &fmt, const Op &op, int r0, 
         const int i = live ? fmt.row(t) : -1;
         const bool own = i >= 0 && lane == 0;
         typename Op::Pre pre;
-        if (own) op.load(i, pre);
+        if (own) {
+            op.early(i, pre);
+            op.load(i, pre);
+        }
         TX s = 0;
-        if (op.need_sum()) s = fmt.template sum<TX, TX>(t, i >= 0, lane, op.x(), Op::kstart);
+        if (op.need_sum()) {
+            typename Fmt::template Head<TX> h;
+            fmt.template head<TX>(t, i >= 0, lane, Op::kstart, h);
+            s = fmt.template tail<TX, TX>(h, op.x());
+        }
         if (own) op.store(i, s, pre);
     }
 }
@@ -77,16 +86,29 @@ __device__ __forceinline__ void rows_pass(const Fmt &fmt, const Op &op, int r0, 
 template <typename TX, typename TV, class Op>
 __device__ __noinline__ void mat_pass(const Mat<TV> &M, const Op &op, int r0, int r1) {
     if (r1 <= r0) return;
-    if (M.sell == 2) {
-        fk::SellFmt<TV, 2> f{M.sp, M.ja, M.a, M.bscale, M.rows};
-        rows_pass<fk::SellFmt<TV, 2>, Op, TX>(f, op, r0, r1);
-        return;
-    }
+#define JX_TAIL_SELL(PP)                                            \
+    {                                                               \
+        fk::SellFmt<TV, PP> f{M.sp, M.ja, M.a, M.bscale, M.rows};   \
+        rows_pass<fk::SellFmt<TV, PP>, Op, TX>(f, op, r0, r1);      \
+    }                                                               \
+    break;
     if (M.sell) {
-        fk::SellFmt<TV> f{M.sp, M.ja, M.a, M.bscale, M.rows};
-        rows_pass<fk::SellFmt<TV>, Op, TX>(f, op, r0, r1);
+        if constexpr (std::is_same<TV, __nv_bfloat16>::value) {
+            fk::SellFmt<TV, 1> f{M.sp, M.ja, M.a, M.bscale, M.rows};
+            rows_pass<fk::SellFmt<TV, 1>, Op, TX>(f, op, r0, r1);
+        } else {
+            switch (M.sell) {
+                case 1: JX_TAIL_SELL(1)
+                case 2: JX_TAIL_SELL(2)
+                case 4: JX_TAIL_SELL(4)
+                case 8: JX_TAIL_SELL(8)
+                case 16: JX_TAIL_SELL(16)
+                default: JX_TAIL_SELL(32)
+            }
+        }
         return;
     }
+#undef JX_TAIL_SELL
 #define JX_TAIL_CSR(VV)                                          \
     {                                                            \
         fk::CsrFmt<VV, TV> f{M.ia, M.ja, M.a, M.bscale, M.perm}; \
@@ -110,10 +132,9 @@ template <typename TX, typename TV>
 __device__ bool smooth(const Level<TX, TV> &L, bool zero, GridBarrier *bar, int *err) {
     if (L.smoother == FS_COLOR_GS) {
         for (int p = 0; p < L.npass; ++p) {
-            const int c = L.pass[p];
-            fk::OpGs<TX> op{L.f, L.dinv, L.u, zero ? 1 : 0};
+            const int c = L.pass[p];  // from a zero iterate the first class' neighbours are the zeros set before
+            fk::OpGs<TX> op{L.f, L.dinv, L.u};
             mat_pass<TX, TV>(L.A, op, L.seg[c], L.seg[c + 1]);
-            zero = false;
             if (!grid_barrier(bar, gridDim.x, err)) return false;
         }
     } else if (L.smoother == FS_L1_JACOBI) {
