@@ -79,11 +79,11 @@ struct DepLaunchScope {
     ~DepLaunchScope() { tl_dep_launch = saved; }
 };
 template <typename... KArgs, typename... Args>
-void launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args &&...args) {
+void launch_dep_smem(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -91,6 +91,10 @@ void launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
     cfg.attrs = at;
     cfg.numAttrs = tl_dep_launch ? 1 : 0;
     JX_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+}
+template <typename... KArgs, typename... Args>
+void launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args &&...args) {
+    launch_dep_smem(kernel, grid, block, 0, s, std::forward<Args>(args)...);
 }
 
 // Device memory cache behind DevBuf.  Blocks are bucketed (powers of two up

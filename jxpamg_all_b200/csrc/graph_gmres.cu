@@ -27,8 +27,8 @@
 // ||w - V h2||^2 = ||w||^2 - ||h2||^2, as in delayed CGS2 (Swirydowicz et al.,
 // 2020).  Flexible: the preconditioned directions z_i are kept and x += Z y.
 // Each pass writes per-block partial sums, which one block per row adds up
-// (reduce_rows_kernel, reduce_rows2_kernel) before the one-thread Arnoldi
-// kernel; the kernels of a step are launched as programmatic dependents.
+// (reduce_rows_kernel, reduce_arnoldi_kernel, whose last block then does the
+// step's scalar part); the kernels of a step are launched as programmatic dependents.
 // Options: the basis and the z_i stored in FP32 (krylov_fp32; every product,
 // norm and update still in FP64), and the second pass taken only where the
 // first cancelled more than half of ||w||^2 (selective_reorth, the Daniel-
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kThreads) scale0_kernel(long long n, const dou
 // dst = V[i] (the preconditioner's input buffer)
 template <typename TB>
 __global__ void __launch_bounds__(kThreads) gather_kernel(long long n, const TB *const *__restrict__ V,
-                                                          const GgState *st, double *__restrict__ dst) {
+                                                          const GgState *st, double *dst) {
     grid_dep_wait();
     const TB *src = V[st->i];
     for (long long e = (long long)blockIdx.x * kThreads + threadIdx.x; e < n; e += (long long)gridDim.x * kThreads)
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kThreads) gather_kernel(long long n, const TB 
 // round_src set, src is replaced by its FP32 rounding too, so that the product A z_i that follows and
 // the update x += Z y use the same direction (a preconditioner with FP32 output needs no rounding).
 template <typename TB>
-__global__ void __launch_bounds__(kThreads) scatter_kernel(long long n, double *__restrict__ src,
+__global__ void __launch_bounds__(kThreads) scatter_kernel(long long n, double *src,
                                                            TB *const *__restrict__ Z, const GgState *st, int round_src) {
     grid_dep_wait();
     TB *dst = Z[st->i];
@@ -249,7 +249,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // sum of row[0..G) over one warp (the result in every lane)
-__device__ __forceinline__ double warp_row_sum(const double *__restrict__ row, int G, int lane) {
+__device__ __forceinline__ double warp_row_sum(const double *row, int G, int lane) {
     double v = 0.0;
     for (int j = lane; j < G; j += 32) v += row[j];
     return warp_sum(v);
@@ -261,8 +261,8 @@ __device__ __forceinline__ double warp_row_sum(const double *__restrict__ row, i
 // memory once at the end.
 template <typename TB>
 __global__ void __launch_bounds__(kThreads) dots_kernel(long long n, const TB *const *__restrict__ V,
-                                                        const GgState *st, const double *__restrict__ w,
-                                                        double *__restrict__ partials) {
+                                                        const GgState *st, const double *w,
+                                                        double *partials) {
     static_assert(kSlice == kThreads * 8, "two quads per thread");
     __shared__ double part[kGgMaxK + 2][kThreads / 32];
     grid_dep_wait();
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kThreads) dots_kernel(long long n, const TB *c
 // ||w||^2, i.e. ||w - V h1||^2 = ||w||^2 - ||h1||^2 > ||w||^2 / 2 (the Daniel-Gragg-Kaufman-Stewart
 // criterion with eta = 1/sqrt(2)): then h2 = h1, h1 = 0 and sig = ||w||^2, so that the Arnoldi and
 // final kernels (which use h1 + h2, sig - ||h2||^2 and w - V h2) finish the step from the first pass.
-__global__ void __launch_bounds__(kRedThreads) reduce_h_kernel(const double *__restrict__ partials, int G,
+__global__ void __launch_bounds__(kRedThreads) reduce_h_kernel(const double *partials, int G,
                                                                GgState *st, GgParams P, GgWork W) {
     __shared__ double ww;
     grid_dep_wait();
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_h_kernel(const double *__r
 
 // h1[k] = sum of partials row k (k <= i), one block per row: the rows are summed side by side
 // (without the selective second pass, which reduce_h_kernel decides on from all of them).
-__global__ void __launch_bounds__(kThreads) reduce_rows_kernel(const double *__restrict__ partials, int G,
+__global__ void __launch_bounds__(kThreads) reduce_rows_kernel(const double *partials, int G,
                                                               GgState *st, GgWork W) {
     __shared__ double sh[32];
     grid_dep_wait();
@@ -380,6 +380,104 @@ __global__ void __launch_bounds__(kThreads) reduce_rows_kernel(const double *__r
     }
 }
 
+// One block: the Hessenberg column of this step, its Givens rotation, the residual estimate, the cycle-end
+// rules and, at a cycle end, y = H^-1 rs.  The block brings the column, the rotations and (at a cycle end) the
+// triangle to shared memory with every load in flight; thread 0 runs the recurrence there.  One thread on the
+// device arrays waits for L2 at each of its O(k) and, at the cycle end, O(k^2) steps.  (With the
+// basis read and written without gather and convert launches: a 1.12 M-cell solve 62.8 -> 61.5 ms.)
+struct ArnoldiSmem {
+    double h[kGgMaxK + 1], c[kGgMaxK], sn[kGgMaxK], rs[kGgMaxK + 1];
+    int end;
+};
+__device__ __forceinline__ void arnoldi_step(GgState *st, const GgParams &P, const GgWork &W, double *norms,
+                                             cudaGraphConditionalHandle h_in, ArnoldiSmem &S, double *tri) {
+    const int K = P.k, m = st->i + 1, i = m;  // steps in this cycle, 1-based as in the reference loop
+    const int tid = threadIdx.x;
+    for (int j = tid; j < m; j += blockDim.x) {
+        const double h2 = __ldcg(W.h2 + j);  // other blocks of this launch may have written them
+        S.h[j] = __ldcg(W.h1 + j) + h2;
+        tri[j] = h2;
+        S.rs[j] = W.rs[j];
+        if (j < m - 1) {
+            S.c[j] = W.c[j];
+            S.sn[j] = W.sn[j];
+        }
+    }
+    __syncthreads();
+    GgState &s = *st;
+    if (tid == 0) {
+        const double sig = __ldcg(&s.sig);  // ||w||^2 after the step's last Gram-Schmidt pass
+        double ss = 0.0;
+        for (int j = 0; j < m; ++j) ss += tri[j] * tri[j];
+        const double t2 = sig - ss;
+        double t = t2 > 0.0 ? sqrt(t2) : 0.0;
+        double *h = S.h;
+        h[m] = t;
+        s.scale = t != 0.0 ? 1.0 / t : 0.0;
+        for (int j = 1; j < i; ++j) {
+            t = h[j - 1];
+            h[j - 1] = S.sn[j - 1] * h[j] + S.c[j - 1] * t;
+            h[j] = -S.sn[j - 1] * t + S.c[j - 1] * h[j];
+        }
+        t = h[i] * h[i];
+        t += h[i - 1] * h[i - 1];
+        double gamma = sqrt(t);
+        if (gamma == 0.0) gamma = 1.e-16;
+        const double c = h[i - 1] / gamma, sn = h[i] / gamma;
+        double rsi = -h[i] * S.rs[i - 1];
+        rsi /= gamma;
+        S.rs[i] = rsi;
+        S.rs[i - 1] = c * S.rs[i - 1];
+        h[i - 1] = sn * h[i] + c * h[i - 1];
+        W.c[i - 1] = c;
+        W.sn[i - 1] = sn;
+        W.rs[i] = rsi;
+        W.rs[i - 1] = S.rs[i - 1];
+        const double r_norm = fabs(rsi);
+        const double conv = r_norm / s.normdown;
+        s.normdown = r_norm;
+        s.iter += 1;
+        norms[s.iter] = r_norm;
+        s.r_norm = r_norm;
+        s.i = i;
+        s.m = m;
+        bool end = i >= K || s.iter >= P.max_iter;
+        if (s.iter > 1 && conv > P.convfac) {
+            s.conv_fail = 1;
+            end = true;
+        }
+        if (r_norm <= s.epsilon && s.iter >= P.min_iter) {
+            s.est_conv = 1;
+            end = true;
+        }
+        S.end = end ? 1 : 0;
+        s.cont = end ? 0 : 1;
+        cudaGraphSetConditional(h_in, end ? 0u : 1u);
+    }
+    __syncthreads();
+    // the rotated column (rows 0 .. m) joins the Hessenberg matrix
+    for (int j = tid; j <= m; j += blockDim.x) W.hh[(long long)j * K + (i - 1)] = S.h[j];
+    if (!S.end) return;
+    // back substitution on the upper triangle, row k at tri[k i ..]; the last column is in S.h
+    for (int e = tid; e < i * i; e += blockDim.x) {
+        const int r = e / i, q = e % i;
+        if (q >= r) tri[e] = q == i - 1 ? S.h[r] : W.hh[(long long)r * K + q];
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double *rs = S.rs;
+        rs[i - 1] = rs[i - 1] / tri[i * i - 1];
+        for (int k = i - 2; k >= 0; --k) {
+            double a = 0.0;
+            for (int j = k + 1; j < i; ++j) a -= tri[k * i + j] * rs[j];
+            a += rs[k];
+            rs[k] = a / tri[k * i + k];
+        }
+    }
+    __syncthreads();
+    for (int j = tid; j < i; j += blockDim.x) W.y[j] = S.rs[j];
+}
+
 // The first update and the second Gram products in one pass over the basis:
 // w -= sum_{k <= i} h[k] V[k], then partial <V[k], w> (k <= i) and <w, w> of
 // the updated w over the block's slice of kSlice2 elements (one quad per thread).
@@ -387,23 +485,44 @@ __global__ void __launch_bounds__(kThreads) reduce_rows_kernel(const double *__r
 // products read it again right after, from L1 / L2, so the basis crosses HBM
 // once (separate update and product kernels would read it twice); the products
 // of two vectors are reduced over the warp together.
-template <typename TB>
+// SMALL (at most kSmallBlocks blocks): every block sums the first products' partials (dots, G per row) for
+// itself, and the last block to finish sums its own pass' and does the step's scalar part: the two reduction
+// launches between the passes took longer than the passes there (with the scalar step above: an 8,000-cell
+// solve 4.13 -> 3.86 ms, twelve 30,000-cell systems at once 18.4 -> 16.6).
+constexpr int kSmallBlocks = 64;
+struct SmallStep {
+    const double *dots;
+    int G;
+    GgParams P;
+    GgWork W;
+    double *norms;
+    cudaGraphConditionalHandle h_in;
+};
+template <typename TB, bool SMALL>
 __global__ void __launch_bounds__(kThreads) update_dots_kernel(long long n, const TB *const *__restrict__ V,
-                                                               const GgState *st, const double *__restrict__ h,
-                                                               double *__restrict__ w, double *__restrict__ partials) {
+                                                               GgState *st, const double *h, double *w,
+                                                               double *partials, SmallStep sm) {
     static_assert(kSlice2 == kThreads * 4, "one quad per thread");
     __shared__ const TB *vs[kGgMaxK + 2];
     __shared__ double hs[kGgMaxK + 2];
     __shared__ double part[kGgMaxK + 2][kThreads / 32];
     grid_dep_wait();
-    if (st->skip) return;  // the selective rule kept the first pass
+    if (!SMALL && st->skip) return;  // the selective rule kept the first pass
     const int m = st->i + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k = threadIdx.x; k < m; k += kThreads) {
         vs[k] = V[k];
-        hs[k] = h[k];
+        if (!SMALL) hs[k] = h[k];
     }
+    if (SMALL)
+        for (int k = warp; k < m; k += kThreads / 32) {
+            const double v = warp_row_sum(sm.dots + (long long)k * sm.G, sm.G, lane);
+            if (lane == 0) {
+                hs[k] = v;
+                if (blockIdx.x == 0) sm.W.h1[k] = v;
+            }
+        }
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long q = (long long)blockIdx.x * (kSlice2 / 4) + threadIdx.x;
     const bool live = 4 * q < n;
     double sv[4] = {0.0, 0.0, 0.0, 0.0};
@@ -464,17 +583,50 @@ __global__ void __launch_bounds__(kThreads) update_dots_kernel(long long n, cons
         for (int qq = 0; qq < kThreads / 32; ++qq) v += part[threadIdx.x][qq];
         partials[(long long)threadIdx.x * gridDim.x + blockIdx.x] = v;
     }
+    if constexpr (SMALL) {
+        __shared__ ArnoldiSmem S;
+        __shared__ int last;
+        extern __shared__ double tri[];  // k x k
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            last = atomicAdd(&st->arrived, 1u) == gridDim.x - 1;
+            if (last) st->arrived = 0;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        const int G = gridDim.x;
+        for (int k = warp; k <= m; k += kThreads / 32) {
+            double v = 0.0;
+            for (int j = lane; j < G; j += 32) v += __ldcg(partials + (long long)k * G + j);
+            v = warp_sum(v);
+            if (lane == 0) {
+                if (k < m) sm.W.h2[k] = v;
+                else st->sig = v;
+            }
+        }
+        __syncthreads();
+        arnoldi_step(st, sm.P, sm.W, sm.norms, sm.h_in, S, tri);
+    }
 }
 
 // The second-pass coefficients h2[k] (k <= i) and ||w||^2 (into st->sig) from the fused update's
-// partials, one block per row; nothing when the selective rule kept the first pass (reduce_h_kernel
-// set them then).
-__global__ void __launch_bounds__(kThreads) reduce_rows2_kernel(const double *__restrict__ partials, int G,
-                                                               GgState *st, GgWork W) {
+// partials, one block per row (none when the selective rule kept the first pass: reduce_h_kernel set them
+// then); the block that finishes last does the step's scalar part.
+__global__ void __launch_bounds__(kThreads) reduce_arnoldi_kernel(const double *partials, int G, GgState *st,
+                                                                 GgParams P, GgWork W, double *norms,
+                                                                 cudaGraphConditionalHandle h_in) {
     __shared__ double sh[32];
+    __shared__ ArnoldiSmem S;
+    __shared__ int last;
+    extern __shared__ double tri[];  // k x k
     grid_dep_wait();
-    if (st->skip) return;
     const int m = st->i + 1, k = blockIdx.x;
+    if (st->skip) {
+        if (k == 0) arnoldi_step(st, P, W, norms, h_in, S, tri);
+        return;
+    }
     if (k > m) return;
     double v = 0.0;
     for (int j = threadIdx.x; j < G; j += kThreads) v += partials[(long long)k * G + j];
@@ -482,84 +634,21 @@ __global__ void __launch_bounds__(kThreads) reduce_rows2_kernel(const double *__
     if (threadIdx.x == 0) {
         if (k < m) W.h2[k] = v;
         else st->sig = v;
+        __threadfence();
+        last = atomicAdd(&st->arrived, 1u) == (unsigned)m;
+        if (last) st->arrived = 0;
     }
-}
-
-// One thread: the Hessenberg column of this step, its Givens rotation, the
-// residual estimate, the cycle-end rules and, at a cycle end, y = H^-1 rs.
-__global__ void arnoldi_kernel(GgState *st, GgParams P, GgWork W, double *__restrict__ norms,
-                               cudaGraphConditionalHandle h_in) {
-    grid_dep_wait();
-    if (threadIdx.x != 0) return;
-    const int i0 = st->i, m = i0 + 1;
-    const double sig = st->sig;  // ||w||^2 after the step's last Gram-Schmidt pass
-    GgState &s = *st;
-    const int K = P.k;
-    double *hh = W.hh, *rs = W.rs, *c = W.c, *sn = W.sn;
-#define HH(r, q) hh[(long long)(r) * K + (q)]
-    double ss = 0.0;
-    for (int j = 0; j < m; ++j) {
-        HH(j, i0) = W.h1[j] + W.h2[j];
-        ss += W.h2[j] * W.h2[j];
-    }
-    const double t2 = sig - ss;
-    double t = t2 > 0.0 ? sqrt(t2) : 0.0;
-    HH(m, i0) = t;
-    s.scale = t != 0.0 ? 1.0 / t : 0.0;
-    const int i = m;  // steps in this cycle, 1-based as in the reference loop
-    for (int j = 1; j < i; ++j) {
-        t = HH(j - 1, i - 1);
-        HH(j - 1, i - 1) = sn[j - 1] * HH(j, i - 1) + c[j - 1] * t;
-        HH(j, i - 1) = -sn[j - 1] * t + c[j - 1] * HH(j, i - 1);
-    }
-    t = HH(i, i - 1) * HH(i, i - 1);
-    t += HH(i - 1, i - 1) * HH(i - 1, i - 1);
-    double gamma = sqrt(t);
-    if (gamma == 0.0) gamma = 1.e-16;
-    c[i - 1] = HH(i - 1, i - 1) / gamma;
-    sn[i - 1] = HH(i, i - 1) / gamma;
-    rs[i] = -HH(i, i - 1) * rs[i - 1];
-    rs[i] /= gamma;
-    rs[i - 1] = c[i - 1] * rs[i - 1];
-    HH(i - 1, i - 1) = sn[i - 1] * HH(i, i - 1) + c[i - 1] * HH(i - 1, i - 1);
-    const double r_norm = fabs(rs[i]);
-    const double conv = r_norm / s.normdown;
-    s.normdown = r_norm;
-    s.iter += 1;
-    norms[s.iter] = r_norm;
-    s.r_norm = r_norm;
-    s.i = i;
-    s.m = m;
-    bool end = i >= K || s.iter >= P.max_iter;
-    if (s.iter > 1 && conv > P.convfac) {
-        s.conv_fail = 1;
-        end = true;
-    }
-    if (r_norm <= s.epsilon && s.iter >= P.min_iter) {
-        s.est_conv = 1;
-        end = true;
-    }
-    if (end) {
-        rs[i - 1] = rs[i - 1] / HH(i - 1, i - 1);
-        for (int k = i - 2; k >= 0; --k) {
-            double a = 0.0;
-            for (int j = k + 1; j < i; ++j) a -= HH(k, j) * rs[j];
-            a += rs[k];
-            rs[k] = a / HH(k, k);
-        }
-        for (int j = 0; j < i; ++j) W.y[j] = rs[j];
-    }
-#undef HH
-    s.cont = end ? 0 : 1;
-    cudaGraphSetConditional(h_in, end ? 0u : 1u);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();  // the other blocks' rows
+    arnoldi_step(st, P, W, norms, h_in, S, tri);
 }
 
 // v_{m} = (w - sum_{k < m} h2[k] V[k]) * scale, skipped at a cycle end; a quad per thread and trip,
 // two basis vectors per step of the sum
 template <typename TB>
 __global__ void __launch_bounds__(kThreads) final_kernel(long long n, TB *const *__restrict__ V,
-                                                         const GgState *st, const double *__restrict__ h,
-                                                         const double *__restrict__ w) {
+                                                         const GgState *st, const double *h, const double *w) {
     __shared__ const TB *vs[kGgMaxK + 2];
     __shared__ double hs[kGgMaxK + 2];
     grid_dep_wait();
@@ -737,7 +826,7 @@ void GraphGmres::prepare(Solver &S) {
     W.h2 = W.h1 + (k + 2);
     W.y = W.h2 + (k + 2);
     W.hh = W.y + k;
-    partials.alloc((size_t)(k + 2) * std::max(G, G2));
+    partials.alloc((size_t)(k + 2) * std::max(G, G2) * 2);  // first and second products' (one launch may read and write)
     norms.alloc((size_t)max_iter + 2);
     summary.alloc(8);
     cin.alloc(nn);
@@ -845,37 +934,61 @@ void GraphGmres::record(Solver &S, cudaStream_t s, double *out) {
         c2 = launch_count();
         JX_CUDA(cudaStreamBeginCaptureToGraph(s2, body_in, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         DepLaunchScope dep(S.prm.dep_launch);  // programmatic edges between the step's kernels
-        if (f32)
-            launch_dep(gather_kernel<float>, dim3(G1), dim3(kThreads), s2, nn, V32, st, cin.get());
-        else
-            launch_dep(gather_kernel<double>, dim3(G1), dim3(kThreads), s2, nn, V, st, cin.get());
-        JX_LAUNCH_CHECK();
-        S.cpr.apply_enqueue(cin.get(), cout.get(), s2);
-        if (f32)
-            launch_dep(scatter_kernel<float>, dim3(G1), dim3(kThreads), s2, nn, cout.get(), Z32, st, 1);
-        else
-            launch_dep(scatter_kernel<double>, dim3(G1), dim3(kThreads), s2, nn, cout.get(), Z, st, 0);
-        JX_LAUNCH_CHECK();
-        bsr_spmv<double, double>(A, 1.0, cout.get(), 0.0, w, kerr, s2, staged);
+        // z_i = M^-1 v_i, kept in Z[i], and w = A z_i.  A preconditioner with an FP32 result reads v_i from the
+        // basis itself and the product reads its result (and stores Z[i]) from there: no copies between.
+        const float *z32 = nullptr;
+        if (!staged && !S.cpr.bilu && nn > 0)
+            z32 = S.cpr.fast->apply_enqueue_basis(f32 ? V32 : nullptr, f32 ? nullptr : V, &st->i, s2);
+        if (z32) {
+            if (f32) bsr_spmv_keep<float>(A, z32, w, Z32, &st->i, s2);
+            else bsr_spmv_keep<double>(A, z32, w, Z, &st->i, s2);
+        } else {
+            if (f32)
+                launch_dep(gather_kernel<float>, dim3(G1), dim3(kThreads), s2, nn, V32, st, cin.get());
+            else
+                launch_dep(gather_kernel<double>, dim3(G1), dim3(kThreads), s2, nn, V, st, cin.get());
+            JX_LAUNCH_CHECK();
+            S.cpr.apply_enqueue(cin.get(), cout.get(), s2);
+            if (f32)
+                launch_dep(scatter_kernel<float>, dim3(G1), dim3(kThreads), s2, nn, cout.get(), Z32, st, 1);
+            else
+                launch_dep(scatter_kernel<double>, dim3(G1), dim3(kThreads), s2, nn, cout.get(), Z, st, 0);
+            JX_LAUNCH_CHECK();
+            bsr_spmv<double, double>(A, 1.0, cout.get(), 0.0, w, kerr, s2, staged);
+        }
         if (f32)
             launch_dep(dots_kernel<float>, dim3(G), dim3(kThreads), s2, nn, V32, st, w, pt);
         else
             launch_dep(dots_kernel<double>, dim3(G), dim3(kThreads), s2, nn, V, st, w, pt);
         JX_LAUNCH_CHECK();
-        if (P.selective)
-            launch_dep(reduce_h_kernel, dim3(1), dim3(kRedThreads), s2, pt, G, st, P, W);
-        else
-            launch_dep(reduce_rows_kernel, dim3(kGgMaxK + 1), dim3(kThreads), s2, pt, G, st, W);
-        JX_LAUNCH_CHECK();
-        if (f32)
-            launch_dep(update_dots_kernel<float>, dim3(G2), dim3(kThreads), s2, nn, V32, st, W.h1, w, pt);
-        else
-            launch_dep(update_dots_kernel<double>, dim3(G2), dim3(kThreads), s2, nn, V, st, W.h1, w, pt);
-        JX_LAUNCH_CHECK();
-        launch_dep(reduce_rows2_kernel, dim3(kGgMaxK + 1), dim3(kThreads), s2, pt, G2, st, W);
-        JX_LAUNCH_CHECK();
-        launch_dep(arnoldi_kernel, dim3(1), dim3(32), s2, st, P, W, norms.get(), h_in);
-        JX_LAUNCH_CHECK();
+        double *pt2 = pt + (size_t)(k + 2) * std::max(G, G2);
+        const size_t tri_bytes = sizeof(double) * (size_t)k * k;
+        if (!P.selective && G2 <= kSmallBlocks) {
+            const SmallStep sm{pt, G, P, W, norms.get(), h_in};
+            if (f32)
+                launch_dep_smem(update_dots_kernel<float, true>, dim3(G2), dim3(kThreads), tri_bytes, s2, nn, V32, st,
+                                W.h1, w, pt2, sm);
+            else
+                launch_dep_smem(update_dots_kernel<double, true>, dim3(G2), dim3(kThreads), tri_bytes, s2, nn, V, st,
+                                W.h1, w, pt2, sm);
+            JX_LAUNCH_CHECK();
+        } else {
+            if (P.selective)
+                launch_dep(reduce_h_kernel, dim3(1), dim3(kRedThreads), s2, pt, G, st, P, W);
+            else
+                launch_dep(reduce_rows_kernel, dim3(k + 1), dim3(kThreads), s2, pt, G, st, W);
+            JX_LAUNCH_CHECK();
+            if (f32)
+                launch_dep(update_dots_kernel<float, false>, dim3(G2), dim3(kThreads), s2, nn, V32, st, W.h1, w, pt,
+                           SmallStep{});
+            else
+                launch_dep(update_dots_kernel<double, false>, dim3(G2), dim3(kThreads), s2, nn, V, st, W.h1, w, pt,
+                           SmallStep{});
+            JX_LAUNCH_CHECK();
+            launch_dep_smem(reduce_arnoldi_kernel, dim3(k + 1), dim3(kThreads), tri_bytes, s2, pt, G2, st, P, W,
+                            norms.get(), h_in);
+            JX_LAUNCH_CHECK();
+        }
         if (f32)
             launch_dep(final_kernel<float>, dim3(Gq), dim3(kThreads), s2, nn, V32, st, W.h2, w);
         else
@@ -953,12 +1066,12 @@ void GraphGmres::orth_native(int m, int reps, const double *w, cudaStream_t s) {
         if (P.selective)
             reduce_h_kernel<<<1, kRedThreads, 0, s>>>(pt, G, st, P, W);
         else
-            reduce_rows_kernel<<<kGgMaxK + 1, kThreads, 0, s>>>(pt, G, st, W);
+            reduce_rows_kernel<<<k + 1, kThreads, 0, s>>>(pt, G, st, W);
         JX_LAUNCH_CHECK();
         if (fp32)
-            update_dots_kernel<float><<<G2, kThreads, 0, s>>>(nn, vptr32.get(), st, W.h1, ww, pt);
+            update_dots_kernel<float, false><<<G2, kThreads, 0, s>>>(nn, vptr32.get(), st, W.h1, ww, pt, SmallStep{});
         else
-            update_dots_kernel<double><<<G2, kThreads, 0, s>>>(nn, vptr.get(), st, W.h1, ww, pt);
+            update_dots_kernel<double, false><<<G2, kThreads, 0, s>>>(nn, vptr.get(), st, W.h1, ww, pt, SmallStep{});
         JX_LAUNCH_CHECK();
         if (fp32)
             final_kernel<float><<<Gq, kThreads, 0, s>>>(nn, vptr32.get(), st, W.h2, ww);

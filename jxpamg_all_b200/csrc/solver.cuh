@@ -188,6 +188,7 @@ struct GgState {
     double b_norm, r_norm, r_norm0, epsilon, normdown, scale, rel;
     double r_cycle;  // true residual norm at the current cycle's start (stall rule)
     double sig;      // ||w||^2 of a step that skips the second pass
+    unsigned arrived;  // blocks that finished the step's last reduction (the last one does the scalar step)
     unsigned long long t_start, t_end;  // device global timer (ns) at the solve's start and end
 };
 struct GgParams {
