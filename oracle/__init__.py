@@ -38,7 +38,7 @@ def build(reference: bool = True, jobs: int = 8) -> None:
     """Compile the restatement; also the reference library when its tree exists."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
     tree = os.environ.get("JXF_REFERENCE_TREE", REF_TREE)
-    if reference and tree and os.path.isdir(tree):
+    if reference and tree and os.path.isdir(os.path.join(tree, "jxfpamg-0220", "csrc")):
         subprocess.run(["make", "-s", "-f", os.path.join(HERE, "ref.mk"), f"REF={tree}", f"-j{jobs}"],
                        check=True, cwd=os.path.dirname(HERE))
 
