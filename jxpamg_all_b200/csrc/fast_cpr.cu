@@ -1095,9 +1095,9 @@ struct FastCpr final : FastCprBase {
                 set_error("stage 2: the iterate and start-value vectors must be 8-byte aligned");
                 throw CudaError{cudaErrorInvalidValue, "stage 2 alignment"};
             }
-            const int grid = div_up(r1 - r0, kThreads);
+            const int grid = div_up(r1 - r0, kThreads), few = (sizeof(TAC) == 4 ? 2 : 1) * sm_count();
 #define JX_HGS_CHUNK(BSV, CHV)                                                                              \
-    launch_dep(grid <= sm_count() ? fk::hgs_chunk<BSV, CHV, TV, TAC, TXV, true>                               \
+    launch_dep(grid <= few ? fk::hgs_chunk<BSV, CHV, TV, TAC, TXV, true>                                      \
                                   : fk::hgs_chunk<BSV, CHV, TV, TAC, TXV, false>,                             \
                dim3(grid), dim3(kThreads), s, r0, r1, M.sp.get(), reinterpret_cast<const unsigned *>(M.ja.get()), a, \
                M.rows.get(), r, z, vtp, w, om, plain, so.save)

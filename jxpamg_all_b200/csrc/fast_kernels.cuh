@@ -702,17 +702,19 @@ constexpr unsigned kChunkColMask = 0x3fffffffu, kChunkEarlier = 1u << 30, kChunk
 // loaded after the entry loop, and for 2x2 blocks the kept in-chunk block is re-read by its slot
 // rather than held (measured on C1: 46.9 -> 41.1 us per sweep with the paired x gathers; C4: 103 ->
 // 79 us).
-// FEW: a colour of at most one block per SM, where nothing hides a row's chain of loads (a colour of 3
-// blocks took as long as one of 147).  The row keeps everything in registers: all six off-diagonal
-// entries of a 7-point row in one batch with the diagonal block, read before the wait; then every gather
-// at once with b and the row's own x, the start values through a selected address in place of a branch per
-// entry; the in-chunk block is held (145,297 2x2 rows in FP64, colours of 147 blocks: 9.9 -> 8.0 us,
-// of 3 blocks: 9.9 -> 7.0).
+// FEW: a colour of at most one block per SM (FP32 arithmetic: two, its registers still let both reside), where
+// nothing hides a row's chain of loads (a colour of 3 blocks took as long as one of 147).  The row keeps
+// everything in registers: all six off-diagonal entries of a 7-point row in one batch with the diagonal block,
+// read before the wait; then every gather at once with b and the row's own x, the start values through a
+// selected address in place of a branch per entry; the in-chunk block is held (145,297 2x2 rows in FP64,
+// colours of 147 blocks: 9.9 -> 8.0 us, of 3 blocks: 9.9 -> 7.0).  Applications with / without it, 2x2 FP32,
+// colours of 275 blocks: 187 / 202 us, of 515: 274 / 269; 3x3 FP32, of 188: 199 / 202, of 375: 269 / 252; 2x2
+// FP64, of 275: 310 / 300.
 template <int BS, int CH, typename TV, typename TA, typename TXV, bool FEW>
-__global__ void __launch_bounds__(256, FEW ? 1 : sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3) hgs_chunk(int r0, int r1, const long long *__restrict__ sp,
-                                                 const unsigned *__restrict__ col, const TV *__restrict__ a,
-                                                 const int *__restrict__ rows, const TXV *b,
-                                                 TXV *x, TXV *vt, TA w, TA omega, int plain, int save) {
+__global__ void __launch_bounds__(256, FEW ? 1 : sizeof(TA) == 4 ? (BS == 2 ? 5 : 4) : 3)
+    hgs_chunk(int r0, int r1, const long long *__restrict__ sp, const unsigned *__restrict__ col,
+              const TV *__restrict__ a, const int *__restrict__ rows, const TXV *b, TXV *x, TXV *vt, TA w, TA omega,
+              int plain, int save) {
     static_assert(32 % CH == 0, "chunks tile the 32-row slices");
     constexpr bool kKeepSlot = BS == 2 && !FEW;  // hold the kept in-chunk block's slot, not its values
     constexpr int NB = FEW ? 6 : BS == 2 ? 4 : 2;  // entries loaded per batch
