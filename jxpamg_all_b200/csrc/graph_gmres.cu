@@ -248,6 +248,19 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// The warp's sums of four values, v[lane >> 3] in lane: two exchanges halve what a lane holds, so four sums take
+// six shuffles and additions where one by one they take twenty (a 1.12 M-cell solve 59.5 -> 57.1 ms, 8,000 cells
+// 3.76 -> 3.74).
+__device__ __forceinline__ double warp_sum4(const double v[4], int lane) {
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const double a = (h16 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
+    const double b = (h16 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
+    double c = (h8 ? b : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+
 // sum of row[0..G) over one warp (the result in every lane)
 __device__ __forceinline__ double warp_row_sum(const double *row, int G, int lane) {
     double v = 0.0;
@@ -257,7 +270,7 @@ __device__ __forceinline__ double warp_row_sum(const double *row, int G, int lan
 
 // Block x: partial <V[k], w> over the x-th slice of kSlice elements for every k <= i.  Each thread
 // keeps its two quads of w in registers and streams the same quads of every basis vector past them,
-// two vectors at a time (eight loads in flight); warps reduce with shuffles and combine through shared
+// four vectors at a time; warps reduce them together with shuffles and combine through shared
 // memory once at the end.
 template <typename TB>
 __global__ void __launch_bounds__(kThreads) dots_kernel(long long n, const TB *const *__restrict__ V,
@@ -272,52 +285,37 @@ __global__ void __launch_bounds__(kThreads) dots_kernel(long long n, const TB *c
     ld4n(w, q1, n, w1);
     const int m = st->i + 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto dot = [&](int k) {
+        double a0[4], a1[4], v = 0.0;
+        ld4n(V[k], q0, n, a0);
+        ld4n(V[k], q1, n, a1);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v = fma(a0[r], w0[r], v);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v = fma(a1[r], w1[r], v);
+        return v;
+    };
     int k = 0;
-    for (; k + 1 < m; k += 2) {
-        double a0[4], a1[4], b0[4], b1[4];
-        ld4n(V[k], q0, n, a0);
-        ld4n(V[k], q1, n, a1);
-        ld4n(V[k + 1], q0, n, b0);
-        ld4n(V[k + 1], q1, n, b1);
-        double sa = 0.0, sb = 0.0;
+    for (; k + 3 < m; k += 4) {
+        const double v[4] = {dot(k), dot(k + 1), dot(k + 2), dot(k + 3)};
+        const double s = warp_sum4(v, lane);
+        if ((lane & 7) == 0) part[k + (lane >> 3)][warp] = s;
+    }
+    // the last vectors, and row m: <w, w> (the selective second pass compares it with the first pass' projection)
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            sa = fma(a0[r], w0[r], sa);
-            sb = fma(b0[r], w0[r], sb);
-        }
+    for (int e = 0; e < 4; ++e) {
+        if (k + e < m) {
+            v[e] = dot(k + e);
+        } else if (k + e == m) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            sa = fma(a1[r], w1[r], sa);
-            sb = fma(b1[r], w1[r], sb);
-        }
-        sa = warp_sum(sa);
-        sb = warp_sum(sb);
-        if (lane == 0) {
-            part[k][warp] = sa;
-            part[k + 1][warp] = sb;
+            for (int r = 0; r < 4; ++r) v[e] = fma(w0[r], w0[r], v[e]);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) v[e] = fma(w1[r], w1[r], v[e]);
         }
     }
-    if (k < m) {
-        double a0[4], a1[4];
-        ld4n(V[k], q0, n, a0);
-        ld4n(V[k], q1, n, a1);
-        double sa = 0.0;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) sa = fma(a0[r], w0[r], sa);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) sa = fma(a1[r], w1[r], sa);
-        sa = warp_sum(sa);
-        if (lane == 0) part[k][warp] = sa;
-    }
-    {  // row m: <w, w> (the selective second pass compares it with the first pass' projection)
-        double sw = 0.0;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) sw = fma(w0[r], w0[r], sw);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) sw = fma(w1[r], w1[r], sw);
-        sw = warp_sum(sw);
-        if (lane == 0) part[m][warp] = sw;
-    }
+    const double s = warp_sum4(v, lane);
+    if ((lane & 7) == 0 && k + (lane >> 3) <= m) part[k + (lane >> 3)][warp] = s;
     __syncthreads();
     if (threadIdx.x <= m) {
         double v = 0.0;
@@ -484,11 +482,12 @@ __device__ __forceinline__ void arnoldi_step(GgState *st, const GgParams &P, con
 // The update reads the quad of every V[k], two vectors at a time, and the
 // products read it again right after, from L1 / L2, so the basis crosses HBM
 // once (separate update and product kernels would read it twice); the products
-// of two vectors are reduced over the warp together.
+// of four vectors are reduced over the warp together.
 // SMALL (at most kSmallBlocks blocks): every block sums the first products' partials (dots, G per row) for
 // itself, and the last block to finish sums its own pass' and does the step's scalar part: the two reduction
 // launches between the passes took longer than the passes there (with the scalar step above: an 8,000-cell
-// solve 4.13 -> 3.86 ms, twelve 30,000-cell systems at once 18.4 -> 16.6).
+// solve 4.13 -> 3.86 ms, twelve 30,000-cell systems at once 18.4 -> 16.6).  The line:
+// solves with / without it at 64,000 unknowns (63 blocks) 5.99 / 6.04 ms, at 128,000 8.00 / 7.77.
 constexpr int kSmallBlocks = 64;
 struct SmallStep {
     const double *dots;
@@ -546,36 +545,34 @@ __global__ void __launch_bounds__(kThreads) update_dots_kernel(long long n, cons
         }
         st4n(w, q, n, sv);
     }
-    for (int k = 0; k <= m; k += 2) {  // uniform trip count: every lane takes part in the shuffles
-        double v0 = 0.0, v1 = 0.0;
+    // every lane takes part in the shuffles, live or not
+    auto dot = [&](int k) {
+        double a[4], v = 0.0;
         if (live) {
-            double a[4], b[4];
-            if (k < m)
-                ld4n(vs[k], q, n, a);
-            else
+            ld4n(vs[k], q, n, a);
 #pragma unroll
-                for (int r = 0; r < 4; ++r) a[r] = sv[r];
-            if (k + 1 < m)
-                ld4n(vs[k + 1], q, n, b);
-            else
-#pragma unroll
-                for (int r = 0; r < 4; ++r) b[r] = k + 1 == m ? sv[r] : 0.0;
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                v0 = fma(a[r], sv[r], v0);
-                v1 = fma(b[r], sv[r], v1);
-            }
+            for (int r = 0; r < 4; ++r) v = fma(a[r], sv[r], v);
         }
+        return v;
+    };
+    int k = 0;
+    for (; k + 3 < m; k += 4) {
+        const double v[4] = {dot(k), dot(k + 1), dot(k + 2), dot(k + 3)};
+        const double s = warp_sum4(v, lane);
+        if ((lane & 7) == 0) part[k + (lane >> 3)][warp] = s;
+    }
+    double v[4] = {0.0, 0.0, 0.0, 0.0};  // the last vectors, and row m: <w, w>
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-        }
-        if (lane == 0) {
-            part[k][warp] = v0;
-            if (k + 1 <= m) part[k + 1][warp] = v1;
+    for (int e = 0; e < 4; ++e) {
+        if (k + e < m) {
+            v[e] = dot(k + e);
+        } else if (k + e == m) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) v[e] = fma(sv[r], sv[r], v[e]);
         }
     }
+    const double s = warp_sum4(v, lane);
+    if ((lane & 7) == 0 && k + (lane >> 3) <= m) part[k + (lane >> 3)][warp] = s;
     __syncthreads();
     if (threadIdx.x <= m) {
         double v = 0.0;
