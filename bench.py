@@ -647,7 +647,7 @@ TRAFFIC_BYTES = {
     ("c1", "stage2/4/chunk4"): 209_080_576,    # hgs_chunk<2,4,float>: 99,779,584 + 109,300,992 (2 colours)
     ("c1", "cheb/A1/4/csr/4"): 103_513_600,    # row_kernel<CsrFmt<4,float>, OpCheb>: mean of 2 launches
     ("c1", "cheb/A1/4/sell"): 108_742_144,     # row_kernel<SellFmt<float>, OpCheb>: mean of 2 launches
-    ("c1", "bsr_spmv/8"): 318_746_624,         # bsr_spmv_direct_kernel<2, double>
+    ("c1", "bsr_spmv/8"): 318_746_624,         # bsr_spmv_slab_kernel<2, double>
     ("c4", "stage2/4/chunk4"): 389_580_032,    # hgs_chunk<3,4,float>: 189,072,128 + 200,507,904 (2 colours)
 }
 
@@ -713,14 +713,16 @@ def roofline_stage2(G, s, stream, value_bytes, cfg="c1"):
 
 def roofline_level(G, stream, level, op, value_bytes, vec_bytes, cfg="c1"):
     """One pass over AMG level `level` (op 1: a Chebyshev step y = c z + D^-1 A x) in the path's storage
-    precision and layout: algorithmic bytes nnz (p_v + 4) + (n + 1) 4 + 4 n p_x (x, z, D^-1 read,
-    y written) / mean launch time (CUDA events on the solver's stream)."""
+    precision and layout: algorithmic bytes nnz (p_v + 4; 2 where the columns are 16-bit) + (n + 1) 4 +
+    4 n p_x (x, z, D^-1 read, y written) / mean launch time (CUDA events on the solver's stream)."""
     from jxpamg_all_b200 import lib
 
     so = lib.load()
     n, _, nnz = G.level_sizes(level, 0)
     sec = _event_time(stream, lambda r: lib.check(so.jxcpr_solver_level_native(G.h, level, op, r)), 20)
-    alg = nnz * (value_bytes + 4) + (n + 1) * 4 + 4 * n * vec_bytes
+    near = any(line.startswith(f"tuned A{level} ") and "16-bit columns" in line
+               for line in G.setup_report().splitlines())
+    alg = nnz * (value_bytes + (2 if near else 4)) + (n + 1) * 4 + 4 * n * vec_bytes
     layout = _layout(G, f"A{level}")
     ty = {8: "double", 4: "float", 2: "bf16"}[value_bytes]
     if layout == "sell":
@@ -729,12 +731,14 @@ def roofline_level(G, stream, level, op, value_bytes, vec_bytes, cfg="c1"):
         fmt = f"SellFmt<{ty}, 2>"  # two lanes per row
     else:
         fmt = f"CsrFmt<{layout.split('/')[-1]}, {ty}>"
+    if near:
+        fmt, layout = fmt[:-1] + ", 16-bit columns>", layout + "/16"
     return _roof(f"AMG level {level} Chebyshev step (row_kernel<{fmt}, OpCheb>, {n} rows, {nnz} entries)",
                  alg, sec, cfg, f"cheb/A{level}/{value_bytes}/{layout}", {"level": level})
 
 
 def roofline_bsr_spmv(d_ia, d_ja, d_a, s, stream, cfg="c1", staged=0):
-    """The FP64 BSR SpMV y = A x of GMRES on the workload's matrix: bsr_spmv_direct_kernel (the solve's
+    """The FP64 BSR SpMV y = A x of GMRES on the workload's matrix: bsr_spmv_slab_kernel (the solve's
     kernel), or with staged = 1 the TMA-staged bsr_spmv_tma_kernel for comparison."""
     import torch
 
@@ -753,7 +757,7 @@ def roofline_bsr_spmv(d_ia, d_ja, d_a, s, stream, cfg="c1", staged=0):
     sec = _event_time(stream, body, 20)
     bs, nb, nnzb, n = s.block_size, s.num_block_rows, s.nnzb, s.n
     alg = nnzb * (bs * bs * 8 + 4) + (nb + 1) * 4 + 2 * n * 8
-    kname = f"bsr_spmv_tma_kernel<{bs}>" if staged else f"bsr_spmv_direct_kernel<{bs}, double>"
+    kname = f"bsr_spmv_tma_kernel<{bs}>" if staged else f"bsr_spmv_slab_kernel<{bs}, double>"
     return _roof(f"BSR SpMV y = A x ({kname}, FP64)", alg, sec, cfg, "bsr_spmv_tma/8" if staged else "bsr_spmv/8")
 
 

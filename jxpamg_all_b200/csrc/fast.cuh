@@ -65,6 +65,8 @@ struct LevelMat {
     DevBuf<int> ia, ja;         // CSR pattern; sliced ELL: columns in ja
     DevBuf<long long> sp;       // sliced ELL: slice offsets (entries)
     DevBuf<int> rows;           // sliced ELL: vector row of each stored row
+    bool near = false;          // sliced ELL: the columns also in j16, as distances from the row
+    DevBuf<unsigned short> j16;
     std::vector<int> seg;
     DevBuf<double> a64;
     DevBuf<float> a32;

@@ -97,12 +97,16 @@ struct CsrFmt {
 // added with shuffles.  rows[t] is the vector row of stored row t (-1: padding row).  Slots are read in
 // batches of NB, a batch ahead of the gathers it feeds; a slice's width is the same for the whole warp,
 // so the batch's last slots are skipped without divergence.
-template <typename TV, int P = 1>
+// TJ = unsigned short: columns stored as their distance from the row's own index (+ kNear, padding: the row
+// itself), for square operators whose entries all lie within it: 2 bytes less per entry.
+constexpr int kNear = 32768;
+template <typename TV, int P = 1, typename TJ = int>
 struct SellFmt {
     static constexpr int V = P;
     static constexpr int NB = sizeof(TV) == 8 ? 4 : 8;  // slots per batch
+    static constexpr bool NEAR = sizeof(TJ) == 2;
     const long long *sp;
-    const int *col;
+    const TJ *col;
     const TV *a;
     const float *bscale;  // BF16 (P = 1): one scale per 32 stored values (one slot of a slice)
     const int *rows;
@@ -110,6 +114,7 @@ struct SellFmt {
     struct Head {
         long long o;  // slot 0 of the virtual row
         int k, w;     // first slot of the sum, the slice's width
+        int base;     // NEAR: what the stored columns are relative to
         int j[NB];
         TA a[NB];
     };
@@ -130,6 +135,7 @@ struct SellFmt {
         h.k = kstart > lane ? (kstart - lane + P - 1) / P : 0;  // first position >= kstart
         h.o = 0;
         h.w = 0;
+        h.base = NEAR && live ? __ldg(rows + t) - kNear : 0;
         if (live) {
             const long long b0 = __ldg(sp + (vt >> 5)), b1 = __ldg(sp + (vt >> 5) + 1);
             h.w = (int)((b1 - b0) >> 5);
@@ -145,7 +151,7 @@ struct SellFmt {
             TA xv[NB];
 #pragma unroll
             for (int q = 0; q < NB; ++q)
-                if (k + q < w) xv[q] = (TA)x[h.j[q]];
+                if (k + q < w) xv[q] = (TA)x[NEAR ? h.base + h.j[q] : h.j[q]];
             TA av[NB];
 #pragma unroll
             for (int q = 0; q < NB; ++q) av[q] = h.a[q];
@@ -1099,6 +1105,27 @@ __global__ void sell_fill_lanes(int nstored, int P, const int *__restrict__ rows
         const long long pp = o + q % P + 32LL * (q / P);
         col[pp] = je;
         val[pp] = cvt_val<TV>(a[d + e], 1.0);
+    }
+}
+
+// The columns of a square sliced ELL (P lanes per row) as distances from the row (SellFmt's TJ = unsigned
+// short), a thread per virtual row.  *far is set where an entry does not lie near enough; padding (value 0,
+// column 0) takes the row itself where column 0 is too far.
+template <typename TV>
+__global__ void sell_near_columns(int nstored, int P, const int *__restrict__ rows, const long long *__restrict__ sp,
+                                  const int *__restrict__ col, const TV *__restrict__ val,
+                                  unsigned short *__restrict__ near, int *__restrict__ far) {
+    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= (long long)nstored * P) return;
+    const int i = rows[v / P];
+    const long long b0 = sp[v >> 5], b1 = sp[(v >> 5) + 1], o = b0 + (v & 31);
+    const int w = (int)((b1 - b0) >> 5);
+    for (int k = 0; k < w; ++k) {
+        const long long p = o + 32LL * k;
+        const long long d = (long long)col[p] - i + kNear;
+        const bool ok = i >= 0 && d >= 0 && d < 65536;
+        near[p] = (unsigned short)(ok ? d : kNear);
+        if (!ok && i >= 0 && !(col[p] == 0 && val[p] == (TV)0)) *far = 1;
     }
 }
 
