@@ -37,8 +37,8 @@ namespace jxcpr {
 namespace {
 // A point of the first pass: its links in its measure's bucket, its measure and state in one 16-byte
 // record, since the greedy touches points in no order a cache could follow (separate arrays: four lines per
-// point instead of one; the pass over 63,504 / 1.12 M 7-point rows: 5.2 -> 4.7 / 263 -> 230 ms).  Buckets hold measures up to twice the largest initial one: a point's measure grows
-// once per row that depends on it.
+// point instead of one; the pass over 63,504 / 1.12 M 7-point rows: 5.2 -> 4.7 / 263 -> 230 ms).  Buckets
+// hold measures up to twice the largest initial one: a point's measure grows once per row that depends on it.
 struct Point {
     int next, prev, measure, cf;
 };

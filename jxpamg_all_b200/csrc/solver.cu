@@ -183,8 +183,8 @@ void CprPrecond::stage2_sweep(const double *r, double *z, cudaStream_t s) {
     }
     const AmgLevel &L0 = *amg.levels[0];
     if (prm.stage2_solver_type == 3) {
-        hsgs_sweep(A, L0.fwd, L0.bwd, blk_fwd, blk_bwd, r, z, vt.get(), hsgs_work.get(), prm.stage2_relax_weight, prm.stage2_omega,
-                   amg.err.get(), s);
+        hsgs_sweep(A, L0.fwd, L0.bwd, blk_fwd, blk_bwd, r, z, vt.get(), hsgs_work.get(), prm.stage2_relax_weight,
+                   prm.stage2_omega, amg.err.get(), s);
         return;
     }
     hgs_sweep(A, L0.fwd, blk_fwd, r, z, L0.fwd.rank.get(), vt.get(), prm.stage2_relax_weight, prm.stage2_omega,
