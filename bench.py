@@ -758,7 +758,7 @@ def roofline_bsr_spmv(d_ia, d_ja, d_a, s, stream, cfg="c1", staged=0):
     sec = _event_time(stream, body, 20)
     bs, nb, nnzb, n = s.block_size, s.num_block_rows, s.nnzb, s.n
     alg = nnzb * (bs * bs * 8 + 4) + (nb + 1) * 4 + 2 * n * 8
-    kname = f"bsr_spmv_tma_kernel<{bs}>" if staged else f"bsr_spmv_slab_kernel<{bs}, double>"
+    kname = f"bsr_spmv_tma_kernel<{bs}>" if staged else f"bsr_spmv_{'slab' if bs == 2 else 'direct'}_kernel<{bs}, double>"
     return _roof(f"BSR SpMV y = A x ({kname}, FP64)", alg, sec, cfg, "bsr_spmv_tma/8" if staged else "bsr_spmv/8")
 
 

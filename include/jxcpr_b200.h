@@ -58,7 +58,7 @@ JXCPR_API int jxcpr_pool_stats(double *out);
  * (jxfpamg-0220/csrc/operation/mvops/seq_bsr_matvec.c:22-140) and the local
  * part of jxf_ParBSRMatrixMatvec (par_bsr_matvec.c:21-221), with the same
  * rounding sequence (bit-identical results).  staged != 0 selects the
- * persistent TMA-staged kernel; 0 the slab kernel.  x and y must be 16-byte
+ * persistent TMA-staged kernel; 0 the slab (2x2 FP64) or direct kernel.  x and y must be 16-byte
  * aligned.
  */
 JXCPR_API int jxcpr_bsr_matvec_dev(int nb, int bs, long long nnzb, const int *ia, const int *ja, const double *a,

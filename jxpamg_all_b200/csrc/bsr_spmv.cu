@@ -9,7 +9,7 @@
 // multiply and add (the library is compiled with --fmad=false), so results
 // are bit-identical to the reference CPU loop.
 //
-// Two kernels: the slab kernel below (staged == 0, the solves' choice) and the persistent TMA kernel.
+// staged == 0, the solves' choice: the slab or the direct kernel below; else the persistent TMA kernel.
 //
 // TMA kernel: a CTA owns a tile of ROWS consecutive block rows, one thread
 // per output component.  The tile's block values and column indices are a
@@ -202,13 +202,12 @@ __global__ void __launch_bounds__(SpmvTileCfg<BS, V>::THREADS)
     }
 }
 
-// Slab kernel (the default): a block of threads owns ROWS consecutive block rows, one thread per output
+// Slab kernel (2x2 FP64 blocks): a block of threads owns ROWS consecutive block rows, one thread per output
 // component, and first copies their blocks -- one contiguous range -- to shared memory with 16-byte
 // asynchronous copies.  Read where they lie, the rows' blocks cost one cache line each: a warp's load of the 16
 // rows' k-th blocks touches 16 lines 224 bytes apart, and the L1's line rate, not the memory, bounds the 2x2
-// product (1.12 M 2x2 rows in FP64: 68.3 us, 0.72 of the copy rate; this kernel 64.3; 125,600 3x3 rows with
-// FP32 values 24.5, now 24.4).  While the copies are in flight the threads read their rows' first columns and gather x:
-// what then bounds a block is the chain row pointer -> column -> x beside the copy.  The copies need no wait
+// product (1.12 M 2x2 rows in FP64: 65.0 us, 0.75 of the copy rate; this kernel 61.7).  While the copies are in
+// flight the threads read their rows' first columns and gather x: what then bounds a block is the chain row pointer -> column -> x beside the copy.  The copies need no wait
 // that could hang, and start before the kernel ahead has finished (no kernel of a solve writes the matrix).  A
 // block whose range does not fit (rows of more than CAP / ROWS blocks in the mean) reads it from global memory.
 // XV: the type x is stored in (float where the caller's vector is FP32; widened before the product).
@@ -379,6 +378,50 @@ __global__ void scale_kernel(long long n, X beta, X *y) {
     if (i < n) y[i] = y[i] * beta;
 }
 
+// Direct kernel: one thread per output component, its row's blocks read where they lie.  Three values of a
+// 3x3 block's row, or FP32 values, fill more of the lines that a warp's loads touch, and the slab's copy then costs
+// more than it saves (slab / this, 1.12 M rows: 3x3 FP64 123 / 111 us, 3x3 FP32 96 / 86, 2x2 FP32 50.4 / 46.8; 2x2
+// FP64 61.7 / 65.0).  x may be what the kernel ahead wrote: plain loads.
+template <int BS, typename V, typename X, typename XV, class Keep>
+__global__ void __launch_bounds__(256)
+    bsr_spmv_direct_kernel(int nb, const int *__restrict__ ia, const int *__restrict__ ja, const V *__restrict__ a,
+                           const XV *x, X *y, int init_mode, X scale_y, X alpha, Keep keep) {
+    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long row = gid / BS;
+    const int comp = (int)(gid % BS);
+    grid_dep_wait();
+    if (row >= nb) return;
+    const int kb = __ldg(ia + row), ke = __ldg(ia + row + 1);
+    const long long oidx = row * BS + comp;
+    if constexpr (!std::is_same<Keep, NoKeep>::value) {
+        using ZT = typename std::remove_reference<decltype(keep.Z[0][0])>::type;
+        keep.Z[*keep.i][oidx] = (ZT)x[oidx];
+    }
+    X acc = row_init<BS, V, X>(y, oidx, init_mode, scale_y);
+    for (int k = kb; k < ke; ++k) {
+        X xv[BS];
+        gather_wide<BS, X, XV>(x, __ldg(ja + k), xv);
+        const V *v = a + (long long)k * (BS * BS) + comp * BS;
+#pragma unroll
+        for (int j = 0; j < BS; ++j) acc = acc + (X)__ldg(v + j) * xv[j];
+    }
+    y[oidx] = (alpha == X(1)) ? acc : acc * alpha;
+}
+
+// staged == 0: the slab kernel for 2x2 FP64 blocks, else the direct one.
+template <int BS, typename V, typename X, typename XV, class Keep>
+static void launch_unstaged(const BsrView<V> &A, const XV *x, X *y, int init_mode, X scale_y, X alpha, Keep keep,
+                            cudaStream_t stream) {
+    if constexpr (BS == 2 && sizeof(V) == 8) {
+        using Cfg = SlabCfg<BS, V>;
+        launch_dep(bsr_spmv_slab_kernel<BS, V, X, XV, Keep>, dim3(div_up(A.nb, Cfg::ROWS)), dim3(Cfg::THREADS), stream,
+                   A.nb, A.ia, A.ja, A.a, x, y, init_mode, scale_y, alpha, keep);
+    } else {
+        launch_dep(bsr_spmv_direct_kernel<BS, V, X, XV, Keep>, dim3(div_up((long long)A.nb * BS, 256)), dim3(256), stream,
+                   A.nb, A.ia, A.ja, A.a, x, y, init_mode, scale_y, alpha, keep);
+    }
+}
+
 template <int BS, typename V, typename X>
 static void launch_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, int *err, cudaStream_t stream,
                         bool staged) {
@@ -406,9 +449,7 @@ static void launch_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, 
         bsr_spmv_tma_kernel<BS, V, X><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(
             A.nb, A.nnzb, A.ia, A.ja, A.a, x, y, init_mode, temp, alpha, err);
     } else {
-        using Cfg = SlabCfg<BS, V>;
-        launch_dep(bsr_spmv_slab_kernel<BS, V, X, X, NoKeep>, dim3(div_up(A.nb, Cfg::ROWS)), dim3(Cfg::THREADS), stream,
-                   A.nb, A.ia, A.ja, A.a, x, y, init_mode, temp, alpha, NoKeep{});
+        launch_unstaged<BS, V, X, X>(A, x, y, init_mode, temp, alpha, NoKeep{}, stream);
     }
     JX_LAUNCH_CHECK();
 }
@@ -428,9 +469,7 @@ template <int BS, typename ZT>
 static void launch_keep(const BsrView<double> &A, const float *x, double *y, ZT *const *Z, const int *i,
                         cudaStream_t stream) {
     if (A.nb == 0) return;
-    using Cfg = SlabCfg<BS, double>;
-    launch_dep(bsr_spmv_slab_kernel<BS, double, double, float, KeepX<ZT>>, dim3(div_up(A.nb, Cfg::ROWS)),
-               dim3(Cfg::THREADS), stream, A.nb, A.ia, A.ja, A.a, x, y, 0, 0.0, 1.0, KeepX<ZT>{Z, i});
+    launch_unstaged<BS, double, double, float>(A, x, y, 0, 0.0, 1.0, KeepX<ZT>{Z, i}, stream);
     JX_LAUNCH_CHECK();
 }
 
