@@ -610,7 +610,8 @@ __global__ void __launch_bounds__(kThreads) update_dots_kernel(long long n, cons
 
 // The second-pass coefficients h2[k] (k <= i) and ||w||^2 (into st->sig) from the fused update's
 // partials, one block per row (none when the selective rule kept the first pass: reduce_h_kernel set them
-// then); the block that finishes last does the step's scalar part.
+// then); the block that finishes last does the step's scalar part.  Every block of the grid is counted, the
+// ones without a row too: the scalar part advances st->i, by which a block tells whether it has a row.
 __global__ void __launch_bounds__(kThreads) reduce_arnoldi_kernel(const double *partials, int G, GgState *st,
                                                                  GgParams P, GgWork W, double *norms,
                                                                  cudaGraphConditionalHandle h_in) {
@@ -620,19 +621,19 @@ __global__ void __launch_bounds__(kThreads) reduce_arnoldi_kernel(const double *
     extern __shared__ double tri[];  // k x k
     grid_dep_wait();
     const int m = st->i + 1, k = blockIdx.x;
-    if (st->skip) {
-        if (k == 0) arnoldi_step(st, P, W, norms, h_in, S, tri);
-        return;
+    if (!st->skip && k <= m) {  // the same in every thread of the block
+        double v = 0.0;
+        for (int j = threadIdx.x; j < G; j += kThreads) v += partials[(long long)k * G + j];
+        v = block_sum(v, sh);
+        if (threadIdx.x == 0) {
+            if (k < m) W.h2[k] = v;
+            else st->sig = v;
+        }
     }
-    if (k > m) return;
-    double v = 0.0;
-    for (int j = threadIdx.x; j < G; j += kThreads) v += partials[(long long)k * G + j];
-    v = block_sum(v, sh);
+    __syncthreads();  // every thread has read the step before the block is counted
     if (threadIdx.x == 0) {
-        if (k < m) W.h2[k] = v;
-        else st->sig = v;
         __threadfence();
-        last = atomicAdd(&st->arrived, 1u) == (unsigned)m;
+        last = atomicAdd(&st->arrived, 1u) == gridDim.x - 1;
         if (last) st->arrived = 0;
     }
     __syncthreads();

@@ -153,6 +153,32 @@ def test_batch_matches_single_graph_solves():
         G.close()
 
 
+@pytest.mark.parametrize("opt", [dict(k_dim=60), dict(k_dim=12, krylov_fp32=1), dict(k_dim=30, selective_reorth=1)],
+                         ids=lambda o: "-".join(f"{k}{v}" for k, v in o.items()))
+def test_batch_of_larger_systems_matches_single_solves(opt):
+    """Systems of more than 64 Gram-Schmidt blocks (65,536 unknowns), whose step reductions are a launch of
+    k_dim + 1 blocks each, of which the last does the scalar part: side by side in a batch those launches
+    overlap other systems', so that a block may start late.  Iterations, residuals and solutions are the
+    single solves', in repeated launches."""
+    systems = [synth.reservoir_system(30, 110, 10 + k, seed=31 + k, phases=2) for k in range(6)]
+    assert all(s.n > 65536 for s in systems)
+    solvers = [make(s, graph_gmres=1, tol=1e-8, **opt) for s in systems]
+    single = [G.solve(s.b) for G, s in zip(solvers, systems)]
+    hist = [G.norms() for G in solvers]
+    B = CprGmresBatch(solvers)
+    for _ in range(3):
+        out = B.solve([s.b for s in systems])
+        for k, (x, it, rel, conv) in enumerate(single):
+            assert conv and out["status"][k] == 0
+            assert out["iterations"][k] == it and out["rel_residual"][k] == rel
+            assert np.array_equal(out["x"][k], x), k
+    B.close()
+    for G, s, h, (x, it, rel, _) in zip(solvers, systems, hist, single):
+        x2, it2, rel2, _ = G.solve(s.b)
+        assert it2 == it and rel2 == rel and np.array_equal(x2, x) and np.array_equal(G.norms(), h)
+        G.close()
+
+
 def test_batch_device_arrays():
     import torch
 
