@@ -93,7 +93,7 @@ struct FastLevel {
     double cheb[3] = {0, 0, 0};  // p(t) = c0 + c1 t + c2 t^2
     double cheb_lo = 0, cheb_hi = 0, lambda_max = 0;
     DevBuf<TX> f, u, r, z, y1, y2;
-    DevBuf<TX> c;        // level 0: correction of repeated stage-1 cycles
+    DevBuf<TX> c, g;     // level 0, stage1_maxit > 1: a further cycle's correction and its right-hand side
 };
 
 struct FastOptions {

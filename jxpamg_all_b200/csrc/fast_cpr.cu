@@ -1008,7 +1008,8 @@ struct FastCpr final : FastCprBase {
         JX_LAUNCH_CHECK();
     }
 
-    // u0 = V-cycle(f0) from a zero initial guess
+    // u0 = V-cycle(f0) from a zero initial guess; f0 is none of the level's work vectors (the cycle writes lv[0]->r
+    // and reads f0 again after it)
     void vcycle_tx(const TX *f0, TX *u0, cudaStream_t s, const Ends &E = Ends()) {
         const int L = (int)lv.size();
         auto F = [&](int l) -> const TX * { return l == 0 ? f0 : lv[l]->f.get(); };
@@ -1025,11 +1026,6 @@ struct FastCpr final : FastCprBase {
             smooth(Lv, F(l), U(l), true, s, pre);
             const int r0 = Lv.skip_class0 ? Lv.A.seg[1] : 0;
             residual(Lv, F(l), U(l), Lv.r.get(), s, r0);
-            if (r0 > 0 && F(l) == Lv.r.get()) {  // a right-hand side that the residual replaces: class 0 too
-                launch_dep(fk::zero_rows<TX>, dim3(div_up(r0, kThreads)), dim3(kThreads), s, r0,
-                           Lv.A.sell ? Lv.A.rows.get() : Lv.A.perm, Lv.r.get());
-                JX_LAUNCH_CHECK();
-            }
             FastLevel<TX> &Nx = *lv[l + 1];
             if (l + 1 < top && Nx.smoother != FS_COLOR_GS) {
                 const bool cheb = Nx.smoother == FS_CHEB;
@@ -1237,8 +1233,8 @@ struct FastCpr final : FastCprBase {
         vcycle_tx(L0.f.get(), L0.u.get(), s, E);
         for (int it = 1; it < cfg.stage1_maxit; ++it) {
             // further AMG iterations as residual corrections: u += V(f - A u)
-            residual(L0, L0.f.get(), L0.u.get(), L0.r.get(), s);
-            vcycle_tx(L0.r.get(), L0.c.get(), s);
+            residual(L0, L0.f.get(), L0.u.get(), L0.g.get(), s);
+            vcycle_tx(L0.g.get(), L0.c.get(), s);
             launch_dep(add_kernel<TX>, dim3(div_up(L0.n, kThreads)), dim3(kThreads), s, L0.n, L0.u.get(),
                        L0.c.get());
             JX_LAUNCH_CHECK();
@@ -1513,7 +1509,10 @@ static FastCprBase *build_fast(Amg &H, const BsrView<double> &A, const CprConfig
             alloc_vec(Lv.r, n);
             Lv.r.zero(s);  // entries no residual writes (class 0 of level 0) meet R's padding: finite
             alloc_vec(Lv.z, n);
-            if (l == 0) alloc_vec(Lv.c, n);
+            if (l == 0 && cfg.stage1_maxit > 1) {
+                alloc_vec(Lv.c, n);
+                alloc_vec(Lv.g, n);
+            }
             const int pk = fp64 ? VAL_F64 : VAL_F32;  // transfer operators: FP32 in the mixed path
             const CsrView<double> Pv = HL.P.view();
             CsrView<double> Rv = HL.R.view();

@@ -334,14 +334,6 @@ __global__ void gs_first_class(int nstored, int cend, const int *__restrict__ ro
     if (i >= 0) u[i] = d != (TX)0 ? f[i] * d : (TX)0;
 }
 
-template <typename TX>
-__global__ void zero_rows(int nstored, const int *__restrict__ rows, TX *r) {
-    grid_dep_wait();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t < nstored ? (rows ? __ldg(rows + t) : t) : -1;
-    if (i >= 0) r[i] = (TX)0;
-}
-
 // The restriction also relaxes the first colour class from a zero iterate where level 0 is smoothed by
 // multicolour Gauss-Seidel: dinv0 (nullptr: not wanted) holds 1 / a_ii on class 0 and 0 elsewhere, and
 // u_i = f_i dinv0_i is what gs_first_class leaves.

@@ -9,6 +9,7 @@ must not change results (CUDA-graph replay) do not.
 """
 import numpy as np
 import pytest
+import scipy.sparse
 
 import oracle
 from jxpamg_all_b200.solver import CprGmres
@@ -306,3 +307,41 @@ def test_two_lane_sliced_ell(precision):
         assert conv and true_rel(s, x) <= 1.05e-6, (lanes, it, rel)
         its[lanes] = it
     assert abs(its[2] - its[1]) <= 2, its
+
+
+@pytest.mark.parametrize("opt,eps", [(dict(precision=0, fast_smoother=0), 2.0 ** -53),
+                                     (dict(precision=0, fast_smoother=1, tail_rows=4000), 2.0 ** -53),
+                                     (dict(precision=1, fast_smoother=1, flexible=1), 2.0 ** -24),
+                                     (dict(precision=3, fast_smoother=0, flexible=1), 2.0 ** -24)],
+                         ids=["fp64", "fp64-cheb-tail", "mixed", "hybrid"])
+@pytest.mark.parametrize("name", ["small", "c0", "three"])
+def test_further_stage1_iterations_correct_the_residual(systems, name, opt, eps):
+    """stage1_maxit = 3 without stage-2 sweeps: the pressure of an application is u <- u + V(f - A_0 u) twice
+    after V(f), with A_0 and V of the same hierarchy (here formed in FP64 from vcycle()).
+
+    The pressure diagonal is raised by a fifth: the Jacobian's is its off-diagonal sum up to the compressibility,
+    and the constant vector, which A_0 then all but annihilates, would bring a residual's rounding back 1e5 times
+    larger.  With it, |A_0| |u| <= 2.2 diag |u| and |A_0^-1 diag| <= 1 / (1 - 1 / 1.2) = 6: a residual of 9 terms,
+    rounded, moves the correction by at most 6 * 2.2 * 9 eps < 120 eps relative to u, twice, and each V-cycle
+    rounds its own passes to no more than the same; 1,000 eps (2e-13, 6e-5) holds them together."""
+    s = synth.reservoir_system(14, 15, 13, 8, phases=3) if name == "three" else systems(name)
+    bs = s.block_size
+    a = s.a.reshape(-1, bs, bs).copy()
+    a[s.ia[:-1], 0, 0] *= 1.2  # the diagonal block is a row's first
+    base = dict(decouple=0, smoother_order=1, coarse_exact=0, stage2_maxit=0, autotune=0, **opt)
+    G = CprGmres(stage1_maxit=3, **base).setup(s.ia, s.ja, a.ravel(), bs)
+    V = CprGmres(stage1_maxit=1, **base).setup(s.ia, s.ja, a.ravel(), bs)
+    ia, ja, av, _ = V.level_matrix(0)
+    assert V.num_levels() > 1
+    A0 = scipy.sparse.csr_matrix((av, ja, ia), shape=(len(ia) - 1,) * 2)
+    r = np.random.default_rng(17).standard_normal(s.n)
+    f = r[::bs].copy()
+    u = V.vcycle(f)
+    for _ in range(2):
+        u = u + V.vcycle(f - A0 @ u)
+    z = G.cpr_apply(r).reshape(-1, bs)
+    assert np.linalg.norm(z[:, 0] - u) <= 1000 * eps * np.linalg.norm(u)
+    assert not np.any(z[:, 1:])
+    assert np.array_equal(G.cpr_apply(r).reshape(-1, bs), z)
+    G.close()
+    V.close()
