@@ -1124,6 +1124,13 @@ __global__ void sell_near_columns(int nstored, int P, const int *__restrict__ ro
     }
 }
 
+// *longest (0 before) = the largest row length
+__global__ void longest_row(int n, const int *__restrict__ ia, int *longest) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int len = __reduce_max_sync(0xffffffffu, i < n ? ia[i + 1] - ia[i] : 0);
+    if ((threadIdx.x & 31) == 0) atomicMax(longest, len);
+}
+
 // The CSR counterpart of sell_fill's `sorted`: each row's entries after the first in ascending column
 // order (the first, the diagonal of a square operator, stays first), by an insertion sort of one
 // thread per row.
