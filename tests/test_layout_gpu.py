@@ -8,6 +8,7 @@ import pytest
 
 from jxpamg_all_b200 import synth
 from jxpamg_all_b200.solver import CprGmres
+from systems_util import with_wells
 
 pytestmark = pytest.mark.gpu
 
@@ -26,28 +27,6 @@ def test_layouts_agree(grid, phases, theta, smoother):
         G.close()
     # sums of at most a few hundred products in another order, a handful of levels and passes
     assert np.linalg.norm(out[0] - out[1]) <= 1e-12 * np.linalg.norm(out[0])
-
-
-def with_wells(s, wells, connections, seed):
-    """The system with `wells` further block rows, each coupled both ways to `connections` random cells."""
-    rng = np.random.default_rng(seed)
-    nb, bs = s.num_block_rows, s.block_size
-    a = s.a.reshape(-1, bs, bs).copy()
-    rows, cols, vals = [np.repeat(np.arange(nb), np.diff(s.ia))], [s.ja], [a]
-    for w in range(nb, nb + wells):
-        cells = np.sort(rng.permutation(nb)[:connections])
-        t = rng.uniform(0.1, 2.1, connections)
-        a[s.ia[cells], 0, 0] += t  # the diagonal block is a row's first
-        off, diag = np.zeros((connections, bs, bs)), np.eye(bs)[None].copy()
-        off[:, 0, 0], diag[0, 0, 0] = -t, 1.001 * t.sum()
-        rows += [[w], np.full(connections, w), cells]
-        cols += [[w], cells, np.full(connections, w)]
-        vals += [diag, off, off]
-    rows, cols, vals = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
-    order = np.lexsort((cols, rows != cols, rows))
-    ia = np.zeros(nb + wells + 1, np.int32)
-    ia[1:] = np.cumsum(np.bincount(rows))
-    return ia, cols[order].astype(np.int32), vals[order].reshape(-1), bs
 
 
 @pytest.mark.parametrize("wells,connections", [(0, 0), (2, 50), (3, 900), (1, 9000)])
