@@ -202,44 +202,35 @@ __global__ void __launch_bounds__(SpmvTileCfg<BS, V>::THREADS)
     }
 }
 
-// Slab kernel (2x2 FP64 blocks): a block of threads owns ROWS consecutive block rows, one thread per output
+// Slab kernel (2x2 FP64 blocks): a block of threads owns kSlabRows consecutive block rows, one thread per output
 // component, and first copies their blocks -- one contiguous range -- to shared memory with 16-byte
 // asynchronous copies.  Read where they lie, the rows' blocks cost one cache line each: a warp's load of the 16
 // rows' k-th blocks touches 16 lines 224 bytes apart, and the L1's line rate, not the memory, bounds the 2x2
 // product (1.12 M 2x2 rows in FP64: 65.0 us, 0.75 of the copy rate; this kernel 61.7).  While the copies are in
-// flight the threads read their rows' first columns and gather x: what then bounds a block is the chain row pointer -> column -> x beside the copy.  The copies need no wait
-// that could hang, and start before the kernel ahead has finished (no kernel of a solve writes the matrix).  A
-// block whose range does not fit (rows of more than CAP / ROWS blocks in the mean) reads it from global memory.
+// flight the threads read their rows' first columns and gather x: what then bounds a block is the chain
+// row pointer -> column -> x beside the copy.  The copies need no wait that could hang, and start before the
+// kernel ahead has finished (no kernel of a solve writes the matrix).  A block whose range does not fit (rows of
+// more than 8 blocks in the mean) reads it from global memory.
 // XV: the type x is stored in (float where the caller's vector is FP32; widened before the product).
-template <int BS, typename V>
-struct SlabCfg {
-    static constexpr int THREADS = BS == 2 ? 256 : 192;
-    static constexpr int ROWS = THREADS / BS;
-    static constexpr int CAP = ROWS * (BS == 2 ? 8 : 7);  // blocks
-    static constexpr int SMEM = (CAP * BS * BS * (int)sizeof(V) + 16 + 15) / 16 * 16;
-};
+constexpr int kSlabThreads = 256, kSlabRows = kSlabThreads / 2;
+constexpr int kSlabCap = kSlabRows * 8;                                   // blocks
+constexpr int kSlabBytes = kSlabCap * 4 * (int)sizeof(double) + 16;       // 16: a range that starts off a boundary
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_addr(dst)), "l"(src) : "memory");
 }
 
-// Copies [src, src + bytes) to dst + (src mod 16); the whole 16-byte pieces asynchronously, the ends in
-// elements of T (src is aligned to T).
-template <int THREADS, typename T>
-__device__ __forceinline__ void slab_copy(unsigned char *dst, const T *src, int count) {
-    const uintptr_t s0 = reinterpret_cast<uintptr_t>(src), s1 = s0 + (uintptr_t)count * sizeof(T);
+// Copies count values from src to dst + (src mod 16); the whole 16-byte pieces asynchronously, the ends value by
+// value (src is aligned to 8).
+__device__ __forceinline__ void slab_copy(unsigned char *dst, const double *src, int count) {
+    const uintptr_t s0 = reinterpret_cast<uintptr_t>(src), s1 = s0 + (uintptr_t)count * sizeof(double);
     const uintptr_t base = s0 & ~(uintptr_t)15, a0 = (s0 + 15) & ~(uintptr_t)15, a1 = s1 & ~(uintptr_t)15;
-    if (a0 >= a1) {  // no whole piece
-        for (int i = threadIdx.x; i < count; i += THREADS)
-            *reinterpret_cast<T *>(dst + (s0 - base) + i * sizeof(T)) = src[i];
-        return;
-    }
-    for (uintptr_t p = a0 + 16 * (uintptr_t)threadIdx.x; p < a1; p += 16 * THREADS)
+    for (uintptr_t p = a0 + 16 * (uintptr_t)threadIdx.x; p < a1; p += 16 * kSlabThreads)
         cp_async16(dst + (p - base), reinterpret_cast<const void *>(p));
-    const int lead = (int)((a0 - s0) / sizeof(T)), trail = (int)((s1 - a1) / sizeof(T));
-    if ((int)threadIdx.x < lead + trail) {
-        const int i = (int)threadIdx.x < lead ? (int)threadIdx.x : count - trail + ((int)threadIdx.x - lead);
-        *reinterpret_cast<T *>(dst + (s0 - base) + i * sizeof(T)) = src[i];
+    // a whole number of blocks: both ends are off a boundary, or neither
+    if (a0 != s0 && threadIdx.x < 2 && count > 0) {
+        const int i = threadIdx.x ? count - 1 : 0;
+        *reinterpret_cast<double *>(dst + (s0 - base) + i * sizeof(double)) = src[i];
     }
 }
 
@@ -259,31 +250,27 @@ __device__ __forceinline__ void gather_wide(const XV *x, int c, X (&xv)[BS]) {
     }
 }
 
-// Row `comp` of block k.  PAIR (2x2 blocks): both values in one load, which needs them on a boundary of
-// their size (the caller's array may start between two).
-template <int BS, bool PAIR, typename V>
-__device__ __forceinline__ void load_block_row(const V *a, long long k, int comp, V (&v)[BS]) {
-    const V *p = a + k * (BS * BS) + comp * BS;
-    if constexpr (PAIR && sizeof(V) == 8) {
+// Row `comp` of 2x2 block k.  PAIR: both values in one load, which needs them on a 16-byte boundary (the
+// caller's array may start off one).
+template <bool PAIR>
+__device__ __forceinline__ void load_block_row(const double *a, long long k, int comp, double (&v)[2]) {
+    const double *p = a + k * 4 + comp * 2;
+    if constexpr (PAIR) {
         const double2 t = *reinterpret_cast<const double2 *>(p);
         v[0] = t.x;
         v[1] = t.y;
-    } else if constexpr (PAIR) {
-        const float2 t = *reinterpret_cast<const float2 *>(p);
-        v[0] = t.x;
-        v[1] = t.y;
     } else {
-#pragma unroll
-        for (int j = 0; j < BS; ++j) v[j] = p[j];
+        v[0] = p[0];
+        v[1] = p[1];
     }
 }
 
 // NB entries of a row: their columns, and the x they name.
-template <int BS, typename X, typename XV>
+template <typename XV>
 struct SlabBatch {
     static constexpr int NB = 4;
     int c[NB];
-    X x[NB][BS];
+    double x[NB][2];
     __device__ __forceinline__ void columns(const int *__restrict__ ja, int k, int ke) {
 #pragma unroll
         for (int t = 0; t < NB; ++t)
@@ -292,24 +279,24 @@ struct SlabBatch {
     __device__ __forceinline__ void gather(const XV *xv, int k, int ke) {
 #pragma unroll
         for (int t = 0; t < NB; ++t)
-            if (k + t < ke) gather_wide<BS, X, XV>(xv, c[t], x[t]);
+            if (k + t < ke) gather_wide<2, double, XV>(xv, c[t], x[t]);
     }
 };
 
 // One component of the row's entries [k, ke), in stored order, vals[0] the value of entry 0 of [kv, ...): the
 // first batch's x is in B.
-template <int BS, bool PAIR, typename V, typename X, typename XV>
-__device__ __forceinline__ X slab_row(X acc, int k, int ke, int kv, const V *vals, const int *__restrict__ ja,
-                                      const XV *x, int comp, SlabBatch<BS, X, XV> &B) {
-    constexpr int NB = SlabBatch<BS, X, XV>::NB;
+template <bool PAIR, typename XV>
+__device__ __forceinline__ double slab_row(double acc, int k, int ke, int kv, const double *vals,
+                                           const int *__restrict__ ja, const XV *x, int comp, SlabBatch<XV> &B) {
+    constexpr int NB = SlabBatch<XV>::NB;
     while (k < ke) {
 #pragma unroll
         for (int t = 0; t < NB; ++t)
             if (k + t < ke) {
-                V v[BS];
-                load_block_row<BS, PAIR>(vals, k - kv + t, comp, v);
+                double v[2];
+                load_block_row<PAIR>(vals, k - kv + t, comp, v);
 #pragma unroll
-                for (int j = 0; j < BS; ++j) acc = acc + (X)v[j] * B.x[t][j];
+                for (int j = 0; j < 2; ++j) acc = acc + v[j] * B.x[t][j];
             }
         k += NB;
         B.columns(ja, k, ke);
@@ -326,50 +313,49 @@ struct KeepX {
 };
 struct NoKeep {};
 
-template <int BS, typename V, typename X, typename XV, class Keep>
-__global__ void __launch_bounds__(SlabCfg<BS, V>::THREADS)
-    bsr_spmv_slab_kernel(int nb, const int *__restrict__ ia, const int *__restrict__ ja, const V *__restrict__ a,
-                         const XV *x, X *y, int init_mode, X scale_y, X alpha, Keep keep) {
-    using Cfg = SlabCfg<BS, V>;
-    __shared__ __align__(16) unsigned char slab[Cfg::SMEM];
-    const int tid = threadIdx.x, comp = tid % BS;
-    const int r0 = blockIdx.x * Cfg::ROWS, r1 = min(nb, r0 + Cfg::ROWS);
-    const int row = r0 + tid / BS;
+template <typename XV, class Keep>
+__global__ void __launch_bounds__(kSlabThreads)
+    bsr_spmv_slab_kernel(int nb, const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ a,
+                         const XV *x, double *y, int init_mode, double scale_y, double alpha, Keep keep) {
+    __shared__ __align__(16) unsigned char slab[kSlabBytes];
+    const int tid = threadIdx.x, comp = tid % 2;
+    const int r0 = blockIdx.x * kSlabRows, r1 = min(nb, r0 + kSlabRows);
+    const int row = r0 + tid / 2;
     const bool live = row < r1;
     const int k0 = __ldg(ia + r0), k1 = __ldg(ia + r1);
     const int kb = live ? __ldg(ia + row) : 0, ke = live ? __ldg(ia + row + 1) : 0;
-    const bool staged = k1 - k0 <= Cfg::CAP;
-    const V *vs = a + (long long)k0 * (BS * BS);
+    const bool staged = k1 - k0 <= kSlabCap;
+    const double *vs = a + (long long)k0 * 4;
     if (staged) {
-        slab_copy<Cfg::THREADS>(slab, vs, (k1 - k0) * (BS * BS));
+        slab_copy(slab, vs, (k1 - k0) * 4);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    SlabBatch<BS, X, XV> B;
+    SlabBatch<XV> B;
     B.columns(ja, kb, ke);
     grid_dep_wait();
     B.gather(x, kb, ke);
-    const long long oidx = (long long)row * BS + comp;
-    X acc = 0;
+    const long long oidx = (long long)row * 2 + comp;
+    double acc = 0;
     if (live) {
         if constexpr (!std::is_same<Keep, NoKeep>::value) {
             using ZT = typename std::remove_reference<decltype(keep.Z[0][0])>::type;
             keep.Z[*keep.i][oidx] = (ZT)x[oidx];
         }
-        acc = row_init<BS, V, X>(y, oidx, init_mode, scale_y);
+        acc = row_init<2, double, double>(y, oidx, init_mode, scale_y);
     }
     if (staged) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (!live) return;
     if (staged) {
-        vs = reinterpret_cast<const V *>(slab + (reinterpret_cast<uintptr_t>(vs) & 15));
-        if (BS == 2 && (reinterpret_cast<uintptr_t>(vs) & (2 * sizeof(V) - 1)) == 0)
-            acc = slab_row<BS, BS == 2, V, X, XV>(acc, kb, ke, k0, vs, ja, x, comp, B);
+        vs = reinterpret_cast<const double *>(slab + (reinterpret_cast<uintptr_t>(vs) & 15));
+        if ((reinterpret_cast<uintptr_t>(vs) & 15) == 0)
+            acc = slab_row<true, XV>(acc, kb, ke, k0, vs, ja, x, comp, B);
         else
-            acc = slab_row<BS, false, V, X, XV>(acc, kb, ke, k0, vs, ja, x, comp, B);
+            acc = slab_row<false, XV>(acc, kb, ke, k0, vs, ja, x, comp, B);
     } else {
-        acc = slab_row<BS, false, V, X, XV>(acc, kb, ke, k0, vs, ja, x, comp, B);
+        acc = slab_row<false, XV>(acc, kb, ke, k0, vs, ja, x, comp, B);
     }
-    y[oidx] = (alpha == X(1)) ? acc : acc * alpha;
+    y[oidx] = alpha == 1.0 ? acc : acc * alpha;
 }
 
 template <typename X>
@@ -413,9 +399,8 @@ template <int BS, typename V, typename X, typename XV, class Keep>
 static void launch_unstaged(const BsrView<V> &A, const XV *x, X *y, int init_mode, X scale_y, X alpha, Keep keep,
                             cudaStream_t stream) {
     if constexpr (BS == 2 && sizeof(V) == 8) {
-        using Cfg = SlabCfg<BS, V>;
-        launch_dep(bsr_spmv_slab_kernel<BS, V, X, XV, Keep>, dim3(div_up(A.nb, Cfg::ROWS)), dim3(Cfg::THREADS), stream,
-                   A.nb, A.ia, A.ja, A.a, x, y, init_mode, scale_y, alpha, keep);
+        launch_dep(bsr_spmv_slab_kernel<XV, Keep>, dim3(div_up(A.nb, kSlabRows)), dim3(kSlabThreads), stream, A.nb, A.ia,
+                   A.ja, A.a, x, y, init_mode, scale_y, alpha, keep);
     } else {
         launch_dep(bsr_spmv_direct_kernel<BS, V, X, XV, Keep>, dim3(div_up((long long)A.nb * BS, 256)), dim3(256), stream,
                    A.nb, A.ia, A.ja, A.a, x, y, init_mode, scale_y, alpha, keep);

@@ -1,6 +1,8 @@
-"""The slab SpMV kernel at its edges, bit-exact against the oracle: arrays that start off 16-byte boundaries
-(the copied range's ends go element by element), blocks of rows whose range just fits its shared memory and
-just does not, empty rows, a last block with few rows."""
+"""The unstaged SpMV kernels at their edges, bit-exact against the oracle: arrays that start off 16-byte
+boundaries, empty rows, a last block with few rows.  2x2 FP64 blocks run the slab kernel, which copies the range
+of 128 rows to shared memory (its ends value by value off a boundary), unless it holds more than 1,024 blocks:
+"fits" and "exceeds" are the two sides.  3x3 blocks and FP32 values run the direct kernel, one thread per
+component, on rows of the same kinds."""
 import numpy as np
 import pytest
 
@@ -9,7 +11,8 @@ from jxpamg_all_b200 import lib
 
 pytestmark = pytest.mark.gpu
 
-# rows per block of threads, blocks its shared memory holds (bs 2, 3)
+# bs 2: the slab kernel's rows per block of threads and the blocks its shared memory holds; bs 3: as many rows
+# of seven blocks
 ROWS, CAP = {2: 128, 3: 64}, {2: 1024, 3: 448}
 
 
@@ -35,7 +38,7 @@ def lengths(kind, bs):
 @pytest.mark.parametrize("kind", ["ragged", "fits", "exceeds"])
 @pytest.mark.parametrize("f32", [False, True])
 @pytest.mark.parametrize("off_a,off_j", [(0, 0), (1, 3), (2, 1), (3, 2)])
-def test_slab_spmv_bit_exact(bs, kind, f32, off_a, off_j):
+def test_unstaged_spmv_bit_exact(bs, kind, f32, off_a, off_j):
     from gpu_util import dev, host, ptr, stream
 
     ia, ja, a, x = pattern(bs, lengths(kind, bs), 7)
