@@ -647,7 +647,7 @@ TRAFFIC_BYTES = {
     ("c1", "stage2/4/chunk4"): 205_356_800,    # hgs_chunk<2,4,float>: 99,701,760 + 105,655,040 (2 colours)
     ("c1", "cheb/A1/4/csr/4"): 103_513_600,    # row_kernel<CsrFmt<4,float>, OpCheb>: mean of 2 launches
     ("c1", "cheb/A1/4/sell"): 108_742_144,     # row_kernel<SellFmt<float>, OpCheb>: mean of 2 launches
-    ("c1", "cheb/A1/4/sell/16"): 80_297_728,   # row_kernel<SellFmt<float, 1, 16-bit>, OpCheb>: mean of 2 launches
+    ("c1", "cheb/A1/4/sell/near"): 80_297_728,  # row_kernel<SellFmt<float, 16-bit columns>, OpCheb>: mean of 2
     ("c1", "bsr_spmv/8"): 314_628_864,         # bsr_spmv_slab_kernel<2, double>
     ("c4", "stage2/4/chunk4"): 389_580_032,    # hgs_chunk<3,4,float>: 189,072,128 + 200,507,904 (2 colours)
 }
@@ -712,6 +712,17 @@ def roofline_stage2(G, s, stream, value_bytes, cfg="c1"):
                  {"sweep_ms": sec * 1e3})
 
 
+def level_format(layout, near, value_bytes):
+    """(kernel format, key) of a level operator's layout as the setup report names it: "sell" (one lane per
+    row), "sell/P" (P lanes) or "csr/V"; near: 16-bit columns."""
+    ty = {8: "double", 4: "float", 2: "bf16"}[value_bytes]
+    kind, _, lanes = layout.partition("/")
+    args = [ty] + ([lanes] if lanes else []) if kind == "sell" else [lanes, ty]
+    fmt = "SellFmt" if kind == "sell" else "CsrFmt"
+    return (f"{fmt}<{', '.join(args + (['16-bit columns'] if near else []))}>",
+            layout + ("/near" if near else ""))
+
+
 def roofline_level(G, stream, level, op, value_bytes, vec_bytes, cfg="c1"):
     """One pass over AMG level `level` (op 1: a Chebyshev step y = c z + D^-1 A x) in the path's storage
     precision and layout: algorithmic bytes nnz (p_v + 4; 2 where the columns are 16-bit) + (n + 1) 4 +
@@ -724,16 +735,7 @@ def roofline_level(G, stream, level, op, value_bytes, vec_bytes, cfg="c1"):
     near = any(line.startswith(f"tuned A{level} ") and "16-bit columns" in line
                for line in G.setup_report().splitlines())
     alg = nnz * (value_bytes + (2 if near else 4)) + (n + 1) * 4 + 4 * n * vec_bytes
-    layout = _layout(G, f"A{level}")
-    ty = {8: "double", 4: "float", 2: "bf16"}[value_bytes]
-    if layout == "sell":
-        fmt = f"SellFmt<{ty}>"
-    elif layout == "sell/2":
-        fmt = f"SellFmt<{ty}, 2>"  # two lanes per row
-    else:
-        fmt = f"CsrFmt<{layout.split('/')[-1]}, {ty}>"
-    if near:
-        fmt, layout = fmt[:-1] + ", 16-bit columns>", layout + "/16"
+    fmt, layout = level_format(_layout(G, f"A{level}"), near, value_bytes)
     return _roof(f"AMG level {level} Chebyshev step (row_kernel<{fmt}, OpCheb>, {n} rows, {nnz} entries)",
                  alg, sec, cfg, f"cheb/A{level}/{value_bytes}/{layout}", {"level": level})
 

@@ -57,3 +57,17 @@ def test_both_arms_print_the_same_config():
     for cfg in ("c1", "c4"):
         args = SimpleNamespace(config=cfg, opt=[])
         assert bench.common_config(cfg, bench.plain_opts(args)) == bench.common_config(cfg, bench.solver_opts(args))
+
+
+def test_level_formats_have_names_of_their_own():
+    """One lane with 16-bit columns, 16 lanes, and CSR do not share a name or a traffic figure's key."""
+    seen = {}
+    for layout in ("sell", "sell/2", "sell/4", "sell/16", "sell/32", "csr/1", "csr/4", "csr/16"):
+        for near in (False, True) if layout in ("sell", "sell/2", "sell/4") else (False,):
+            for name in bench.level_format(layout, near, 4):
+                assert name not in seen, (name, seen[name])
+                seen[name] = (layout, near)
+    assert bench.level_format("sell", True, 4) == ("SellFmt<float, 16-bit columns>", "sell/near")
+    assert bench.level_format("sell/16", False, 8) == ("SellFmt<double, 16>", "sell/16")
+    assert bench.level_format("csr/4", False, 4) == ("CsrFmt<4, float>", "csr/4")
+    assert ("c1", "cheb/A1/4/sell/near") in bench.TRAFFIC_BYTES
