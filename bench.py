@@ -644,12 +644,12 @@ def other_workloads(args):
 # dram__bytes_write.sum; layouts reused through JXCPR_TUNE_CACHE), each summarised in profiles/:
 # (workload, kernel key) -> bytes.  None where not captured.
 TRAFFIC_BYTES = {
-    ("c1", "stage2/4/chunk4"): 205_356_800,    # hgs_chunk<2,4,float>: 99,701,760 + 105,655,040 (2 colours)
+    ("c1", "stage2/4/chunk4"): 207_780_864,    # hgs_chunk<2,4,float>: 99,497,984 + 108,282,880 (2 colours)
     ("c1", "cheb/A1/4/csr/4"): 103_513_600,    # row_kernel<CsrFmt<4,float>, OpCheb>: mean of 2 launches
     ("c1", "cheb/A1/4/sell"): 108_742_144,     # row_kernel<SellFmt<float>, OpCheb>: mean of 2 launches
-    ("c1", "cheb/A1/4/sell/near"): 80_297_728,  # row_kernel<SellFmt<float, 16-bit columns>, OpCheb>: mean of 2
-    ("c1", "bsr_spmv/8"): 314_628_864,         # bsr_spmv_slab_kernel<2, double>
-    ("c4", "stage2/4/chunk4"): 389_580_032,    # hgs_chunk<3,4,float>: 189,072,128 + 200,507,904 (2 colours)
+    ("c1", "cheb/A1/4/sell/near"): 82_076_416,  # row_kernel<SellFmt<float, 16-bit columns>, OpCheb>: mean of 2
+    ("c1", "bsr_spmv/8"): 317_666_304,         # bsr_spmv_slab_kernel<double, NoKeep>
+    ("c4", "stage2/4/chunk4"): 389_371_648,    # hgs_chunk<3,4,float>: 189,119,232 + 200,252,416 (2 colours)
 }
 
 
