@@ -264,38 +264,42 @@ def common_config(cfg, opts):
 
 def reference_full_solve(s, threads, cfg):
     """One complete run of the reference library on the host: decoupling, CPR setup and GMRES to
-    FP64 rel-res 1e-6.  Returns (seconds per phase [decouple, setup, solve], iterations, kind)."""
+    FP64 rel-res 1e-6.  Returns (seconds per phase [decouple, setup, solve], iterations)."""
     os.environ["OMP_NUM_THREADS"] = str(threads)
     import oracle
 
     dec = CONFIG_OPTS.get(cfg, {}).get("decouple", 1)
     kd = CONFIG_OPTS.get(cfg, {}).get("k_dim", 30)
     mi = CONFIG_OPTS.get(cfg, {}).get("max_iter", 300)
+    r = oracle.ref_gmres(s.ia, s.ja, s.a, s.block_size, s.b, decouple=dec, tol=1e-6, max_iter=mi, k_dim=kd)
+    if not r["converged"]:
+        raise RuntimeError(f"reference solve did not converge (rel {r['rel']})")
+    return [float(r["times"][0]), float(r["times"][1]), float(r["times"][2])], r["iters"]
+
+
+def reference_unavailable():
+    """Prints the reference arm's line and returns True where the reference library is not built: the arm
+    runs the reference or nothing."""
+    import oracle
+
     if oracle.ref_available():
-        r = oracle.ref_gmres(s.ia, s.ja, s.a, s.block_size, s.b, decouple=dec, tol=1e-6, max_iter=mi, k_dim=kd)
-        if not r["converged"]:
-            raise RuntimeError(f"reference solve did not converge (rel {r['rel']})")
-        return [float(r["times"][0]), float(r["times"][1]), float(r["times"][2])], r["iters"], "reference"
-    t0 = time.perf_counter()
-    a, b = oracle.bsr_decouple(s.ia, s.ja, s.a, s.block_size, s.b, dec)
-    t1 = time.perf_counter()
-    C = oracle.OracleCPR(s.ia, s.ja, a, s.block_size)
-    t2 = time.perf_counter()
-    r = oracle.gmres(s.ia, s.ja, a, s.block_size, b, tol=1e-6, max_iter=mi, cpr=C, k_dim=kd)
-    t3 = time.perf_counter()
-    return [t1 - t0, t2 - t1, t3 - t2], r["iters"], "port"
+        return False
+    print(json.dumps({"impl": "reference",
+                      "unavailable": "the reference library is not built: no source tree to compile it from"}),
+          flush=True)
+    return True
 
 
 def run_reference(args):
     """--impl reference: the reference's own CPU implementation of the path (compiled from its sources
-    into oracle/_ref; the oracle restatement where it is absent) on all host threads.  Each timed step is
+    into oracle/_ref; where it is absent the line says "unavailable") on all host threads.  Each timed step is
     one complete run to convergence; value = the GMRES solve phase (setup excluded, as in our arm's
     value), e2e = decoupling + CPR setup + solve (as our arm's e2e, which also includes the uploads).
     Warm-up steps are short runs (two GMRES iterations) that page the library and the system in.  A
     complete run takes about 35 s on C1 and 250 s on C4, so the timed runs stop once REF_BUDGET_S
     has passed (at least one): the line's `steps` is the number of runs made."""
     ws, rank, _ = dist_env()
-    if rank != 0:
+    if rank != 0 or reference_unavailable():
         return 0
     from jxpamg_all_b200 import synth
 
@@ -307,12 +311,11 @@ def run_reference(args):
     dec = CONFIG_OPTS.get(args.config, {}).get("decouple", 1)
     kd = CONFIG_OPTS.get(args.config, {}).get("k_dim", 30)
     for _ in range(args.warmup):
-        if oracle.ref_available():
-            oracle.ref_gmres(s.ia, s.ja, s.a, s.block_size, s.b, decouple=dec, tol=1e-6, max_iter=2, k_dim=kd)
-    phases, iters, kind = [], [], None
+        oracle.ref_gmres(s.ia, s.ja, s.a, s.block_size, s.b, decouple=dec, tol=1e-6, max_iter=2, k_dim=kd)
+    phases, iters = [], []
     w0 = time.perf_counter()
     for _ in range(args.steps):
-        t, it, kind = reference_full_solve(s, threads, args.config)
+        t, it = reference_full_solve(s, threads, args.config)
         phases.append(t)
         iters.append(it)
         if time.perf_counter() - w0 > REF_BUDGET_S:
@@ -321,9 +324,7 @@ def run_reference(args):
     ph = np.array(phases)
     value = float(ph[:, 2].mean())
     total = float(ph.sum(axis=1).mean())
-    what = ("reference JXFPAMG built from source (FP64)" if kind == "reference"
-            else "oracle C restatement (FP64, the reference library was not built)")
-    desc = (f"{what}, {threads} OpenMP threads, {len(phases)} complete runs to FP64 rel-res 1e-6 "
+    desc = (f"reference JXFPAMG built from source (FP64), {threads} OpenMP threads, {len(phases)} complete runs to FP64 rel-res 1e-6 "
             f"({iters[0]} GMRES iterations; decoupling {ph[:, 0].mean():.2f} s, CPR setup {ph[:, 1].mean():.2f} s, "
             f"solve {value:.2f} s per run; {wall:.0f} s in all)")
     line = {
@@ -337,7 +338,7 @@ def run_reference(args):
                                         "reported in e2e)",
                     "iterations": iters[0], "decouple_s": float(ph[:, 0].mean()), "setup_s": float(ph[:, 1].mean()),
                     "solve_s": value, "ms_per_step_definition": "one complete run (decoupling + setup + solve)"},
-        "cpu_baseline": {"value": value, "unit": UNIT, "cores": threads, "kind": kind, "sample": desc},
+        "cpu_baseline": {"value": value, "unit": UNIT, "cores": threads, "kind": "reference", "sample": desc},
         "e2e": {"value": total, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
     print(json.dumps(line), flush=True)
@@ -855,7 +856,7 @@ def batch_reference_sample(systems, threads):
 
 def run_batch_reference(args):
     ws, rank, _ = dist_env()
-    if rank != 0:
+    if rank != 0 or reference_unavailable():
         return 0
     from jxpamg_all_b200 import synth
 

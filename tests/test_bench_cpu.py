@@ -6,9 +6,12 @@ three-phase C4 True-IMPES, GMRES(60), the plain CPR weights and no learned
 model; the plain FP64 path always keeps the reference CPR's weights and its
 host-driven GMRES.
 """
+import json
 import os
 import sys
 from types import SimpleNamespace
+
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
@@ -71,3 +74,15 @@ def test_level_formats_have_names_of_their_own():
     assert bench.level_format("sell/16", False, 8) == ("SellFmt<double, 16>", "sell/16")
     assert bench.level_format("csr/4", False, 4) == ("CsrFmt<4, float>", "csr/4")
     assert ("c1", "cheb/A1/4/sell/near") in bench.TRAFFIC_BYTES
+
+
+@pytest.mark.parametrize("config", ["c1", "c3"])
+def test_reference_arm_without_the_reference_library(config, monkeypatch, capsys):
+    """The arm runs the reference or says that it cannot: never this repository's own code."""
+    import oracle
+
+    monkeypatch.setattr(oracle, "ref_available", lambda: False)
+    args = SimpleNamespace(config=config, gpus=1, steps=2, warmup=1)
+    assert (bench.run_batch_reference if config == "c3" else bench.run_reference)(args) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
