@@ -206,12 +206,13 @@ __global__ void __launch_bounds__(SpmvTileCfg<BS, V>::THREADS)
 // component, and first copies their blocks -- one contiguous range -- to shared memory with 16-byte
 // asynchronous copies.  Read where they lie, the rows' blocks cost one cache line each: a warp's load of the 16
 // rows' k-th blocks touches 16 lines 224 bytes apart, and the L1's line rate, not the memory, bounds the 2x2
-// product (1.12 M 2x2 rows in FP64: 65.0 us, 0.75 of the copy rate; this kernel 60.7 with six blocks per SM, 63.0
-// with the five that 48 registers leave).  While the copies are in flight the threads read their rows' first
-// columns and gather x: what then bounds a block is the chain row pointer -> column -> x beside the copy.  The
-// copies need no wait that could hang, and start before the kernel ahead has finished (no kernel of a solve
-// writes the matrix).  A block whose range does not fit (rows of more than 8 blocks in the mean) reads it from
-// global memory.
+// product (1.12 M 2x2 rows in FP64: 65.0 us, 0.75 of the copy rate; this kernel 63.0).  While the copies are in
+// flight the threads read their rows' first columns and gather x: what then bounds a block is the chain
+// row pointer -> column -> x beside the copy.  Five blocks of it fit an SM, by its registers (44 to 48).  Held to 40
+// and six blocks it takes 60.7 us alone, but 64 systems solved at once 91.4 ms in place of 82.2 (85.7 with six
+// blocks in the restarts' products only): beside other kernels its shared memory counts.  The copies need no
+// wait that could hang, and start before the kernel ahead has finished (no kernel of a solve writes the matrix).  A
+// block whose range does not fit (rows of more than 8 blocks in the mean) reads it from global memory.
 // XV: the type x is stored in (float where the caller's vector is FP32; widened before the product).
 constexpr int kSlabThreads = 256, kSlabRows = kSlabThreads / 2;
 constexpr int kSlabCap = kSlabRows * 8;                                   // blocks
@@ -315,7 +316,7 @@ struct KeepX {
 struct NoKeep {};
 
 template <typename XV, class Keep>
-__global__ void __launch_bounds__(kSlabThreads, 6)
+__global__ void __launch_bounds__(kSlabThreads)
     bsr_spmv_slab_kernel(int nb, const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ a,
                          const XV *x, double *y, int init_mode, double scale_y, double alpha, Keep keep) {
     __shared__ __align__(16) unsigned char slab[kSlabBytes];
@@ -368,7 +369,7 @@ __global__ void scale_kernel(long long n, X beta, X *y) {
 // Direct kernel: one thread per output component, its row's blocks read where they lie.  Three values of a
 // 3x3 block's row, or FP32 values, fill more of the lines that a warp's loads touch, and the slab's copy then costs
 // more than it saves (slab / this, 1.12 M rows: 3x3 FP64 123 / 111 us, 3x3 FP32 96 / 86, 2x2 FP32 50.4 / 46.8; 2x2
-// FP64 60.7 / 65.0).  x may be what the kernel ahead wrote: plain loads.
+// FP64 63.0 / 65.0).  x may be what the kernel ahead wrote: plain loads.
 template <int BS, typename V, typename X, typename XV, class Keep>
 __global__ void __launch_bounds__(256)
     bsr_spmv_direct_kernel(int nb, const int *__restrict__ ia, const int *__restrict__ ja, const V *__restrict__ a,
