@@ -79,14 +79,20 @@ struct CsrFmt {
         if (h.k < h.e) s0 = h.a0 * (TA)x[h.j0];
         if (h.k + V < h.e) s1 = h.a1 * (TA)x[h.j1];
         int k = h.k + 2 * V;
-        // asked for: with the head split off, the compiler no longer unrolls it by itself in every operation (an
-        // l1-Jacobi pass over 23,986 FP64 rows, the longest of 8,601 entries: 153 us unrolled, 264 not)
-#pragma unroll 4
-        for (; k + V < h.e; k += 2 * V) {
+        auto trip = [&]() {
             const int j0 = __ldg(ja + k), j1 = __ldg(ja + k + V);
             const TA a0 = (TA)ldvs(a, bscale, k), a1 = (TA)ldvs(a, bscale, k + V);
             s0 = fma(a0, (TA)x[j0], s0);
             s1 = fma(a1, (TA)x[j1], s1);
+        };
+        // Asked for: with the head split off, the compiler no longer unrolls it by itself in every operation (an
+        // l1-Jacobi pass over 23,986 FP64 rows, the longest of 8,601 entries: 153 us unrolled, 264 not).  One lane
+        // per row is for short rows, two or three trips (64 systems at once: 81.6 ms, 81.8 with it).
+        if constexpr (V > 1) {
+#pragma unroll 4
+            for (; k + V < h.e; k += 2 * V) trip();
+        } else {
+            for (; k + V < h.e; k += 2 * V) trip();
         }
         if (k < h.e) s0 = fma((TA)ldvs(a, bscale, k), (TA)x[__ldg(ja + k)], s0);
         return group_sum<V, TA>(s0 + s1);
