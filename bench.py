@@ -649,7 +649,7 @@ TRAFFIC_BYTES = {
     ("c1", "cheb/A1/4/csr/4"): 103_513_600,    # row_kernel<CsrFmt<4,float>, OpCheb>: mean of 2 launches
     ("c1", "cheb/A1/4/sell"): 108_742_144,     # row_kernel<SellFmt<float>, OpCheb>: mean of 2 launches
     ("c1", "cheb/A1/4/sell/near"): 82_076_416,  # row_kernel<SellFmt<float, 16-bit columns>, OpCheb>: mean of 2
-    ("c1", "bsr_spmv/8"): 317_600_512,         # bsr_spmv_slab_kernel<double, NoKeep>
+    ("c1", "bsr_spmv/8"): 317_666_304,         # bsr_spmv_slab_kernel<double, NoKeep, true>
     ("c4", "stage2/4/chunk4"): 389_371_648,    # hgs_chunk<3,4,float>: 189,119,232 + 200,252,416 (2 colours)
 }
 

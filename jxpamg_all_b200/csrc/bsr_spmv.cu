@@ -206,11 +206,12 @@ __global__ void __launch_bounds__(SpmvTileCfg<BS, V>::THREADS)
 // component, and first copies their blocks -- one contiguous range -- to shared memory with 16-byte
 // asynchronous copies.  Read where they lie, the rows' blocks cost one cache line each: a warp's load of the 16
 // rows' k-th blocks touches 16 lines 224 bytes apart, and the L1's line rate, not the memory, bounds the 2x2
-// product (1.12 M 2x2 rows in FP64: 65.0 us, 0.75 of the copy rate; this kernel 63.0).  While the copies are in
+// product (1.12 M 2x2 rows in FP64: 65.0 us, 0.75 of the copy rate; this kernel 61).  While the copies are in
 // flight the threads read their rows' first columns and gather x: what then bounds a block is the chain
-// row pointer -> column -> x beside the copy.  Five blocks of it fit an SM, by its registers (44 to 48).  Held to 40
-// and six blocks it takes 60.7 us alone, but 64 systems solved at once 91.4 ms in place of 82.2 (85.7 with six
-// blocks in the restarts' products only): beside other kernels its shared memory counts.  The copies need no
+// row pointer -> column -> x beside the copy.  ALONE, the product that a caller asks for by itself, is held to 40
+// registers and six blocks per SM (60.7 us, with five 63.0).  Inside a solve five run (44 to 48 registers): a
+// solve is the same with either, but of 64 systems at once other kernels run beside it, and its shared
+// memory counts (82.2 ms; 85.7 with six blocks in the restarts' products, 91.4 in all).  The copies need no
 // wait that could hang, and start before the kernel ahead has finished (no kernel of a solve writes the matrix).  A
 // block whose range does not fit (rows of more than 8 blocks in the mean) reads it from global memory.
 // XV: the type x is stored in (float where the caller's vector is FP32; widened before the product).
@@ -315,8 +316,9 @@ struct KeepX {
 };
 struct NoKeep {};
 
-template <typename XV, class Keep>
-__global__ void __launch_bounds__(kSlabThreads)
+// ALONE: see above (0: no bound of its own).
+template <typename XV, class Keep, bool ALONE>
+__global__ void __launch_bounds__(kSlabThreads, ALONE ? 6 : 0)
     bsr_spmv_slab_kernel(int nb, const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ a,
                          const XV *x, double *y, int init_mode, double scale_y, double alpha, Keep keep) {
     __shared__ __align__(16) unsigned char slab[kSlabBytes];
@@ -369,7 +371,7 @@ __global__ void scale_kernel(long long n, X beta, X *y) {
 // Direct kernel: one thread per output component, its row's blocks read where they lie.  Three values of a
 // 3x3 block's row, or FP32 values, fill more of the lines that a warp's loads touch, and the slab's copy then costs
 // more than it saves (slab / this, 1.12 M rows: 3x3 FP64 123 / 111 us, 3x3 FP32 96 / 86, 2x2 FP32 50.4 / 46.8; 2x2
-// FP64 63.0 / 65.0).  x may be what the kernel ahead wrote: plain loads.
+// FP64 61 / 65.0).  x may be what the kernel ahead wrote: plain loads.
 template <int BS, typename V, typename X, typename XV, class Keep>
 __global__ void __launch_bounds__(256)
     bsr_spmv_direct_kernel(int nb, const int *__restrict__ ia, const int *__restrict__ ja, const V *__restrict__ a,
@@ -399,10 +401,13 @@ __global__ void __launch_bounds__(256)
 // staged == 0: the slab kernel for 2x2 FP64 blocks, else the direct one.
 template <int BS, typename V, typename X, typename XV, class Keep>
 static void launch_unstaged(const BsrView<V> &A, const XV *x, X *y, int init_mode, X scale_y, X alpha, Keep keep,
-                            cudaStream_t stream) {
+                            cudaStream_t stream, bool alone = false) {
     if constexpr (BS == 2 && sizeof(V) == 8) {
-        launch_dep(bsr_spmv_slab_kernel<XV, Keep>, dim3(div_up(A.nb, kSlabRows)), dim3(kSlabThreads), stream, A.nb, A.ia,
-                   A.ja, A.a, x, y, init_mode, scale_y, alpha, keep);
+        auto kernel = bsr_spmv_slab_kernel<XV, Keep, false>;
+        if constexpr (std::is_same<Keep, NoKeep>::value)
+            if (alone) kernel = bsr_spmv_slab_kernel<XV, Keep, true>;
+        launch_dep(kernel, dim3(div_up(A.nb, kSlabRows)), dim3(kSlabThreads), stream, A.nb, A.ia, A.ja, A.a, x, y,
+                   init_mode, scale_y, alpha, keep);
     } else {
         launch_dep(bsr_spmv_direct_kernel<BS, V, X, XV, Keep>, dim3(div_up((long long)A.nb * BS, 256)), dim3(256), stream,
                    A.nb, A.ia, A.ja, A.a, x, y, init_mode, scale_y, alpha, keep);
@@ -411,7 +416,7 @@ static void launch_unstaged(const BsrView<V> &A, const XV *x, X *y, int init_mod
 
 template <int BS, typename V, typename X>
 static void launch_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, int *err, cudaStream_t stream,
-                        bool staged) {
+                        bool staged, bool alone) {
     const long long n = (long long)A.nb * BS;
     if (A.nb == 0) return;
     if (alpha == X(0)) {
@@ -436,16 +441,17 @@ static void launch_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, 
         bsr_spmv_tma_kernel<BS, V, X><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(
             A.nb, A.nnzb, A.ia, A.ja, A.a, x, y, init_mode, temp, alpha, err);
     } else {
-        launch_unstaged<BS, V, X, X>(A, x, y, init_mode, temp, alpha, NoKeep{}, stream);
+        launch_unstaged<BS, V, X, X>(A, x, y, init_mode, temp, alpha, NoKeep{}, stream, alone);
     }
     JX_LAUNCH_CHECK();
 }
 
 template <typename V, typename X>
-void bsr_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, int *err, cudaStream_t stream, bool staged) {
+void bsr_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, int *err, cudaStream_t stream, bool staged,
+              bool alone) {
     switch (A.bs) {
-        case 2: launch_spmv<2, V, X>(A, alpha, x, beta, y, err, stream, staged); break;
-        case 3: launch_spmv<3, V, X>(A, alpha, x, beta, y, err, stream, staged); break;
+        case 2: launch_spmv<2, V, X>(A, alpha, x, beta, y, err, stream, staged, alone); break;
+        case 3: launch_spmv<3, V, X>(A, alpha, x, beta, y, err, stream, staged, alone); break;
         default:
             set_error("bsr_spmv: unsupported block size %d", A.bs);
             throw CudaError{cudaErrorInvalidValue, "block size"};
@@ -472,10 +478,10 @@ template void bsr_spmv_keep<float>(const BsrView<double> &, const float *, doubl
 template void bsr_spmv_keep<double>(const BsrView<double> &, const float *, double *, double *const *, const int *,
                                     cudaStream_t);
 template void bsr_spmv<double, double>(const BsrView<double> &, double, const double *, double, double *, int *,
-                                       cudaStream_t, bool);
+                                       cudaStream_t, bool, bool);
 template void bsr_spmv<float, double>(const BsrView<float> &, double, const double *, double, double *, int *,
-                                      cudaStream_t, bool);
+                                      cudaStream_t, bool, bool);
 template void bsr_spmv<float, float>(const BsrView<float> &, float, const float *, float, float *, int *,
-                                     cudaStream_t, bool);
+                                     cudaStream_t, bool, bool);
 
 }  // namespace jxcpr

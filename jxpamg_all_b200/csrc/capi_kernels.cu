@@ -75,7 +75,7 @@ int jxcpr_bsr_matvec_dev(int nb, int bs, long long nnzb, const int *ia, const in
     return guarded([&] {
         BsrView<double> A{nb, bs, nnzb, ia, ja, a};
         bsr_spmv<double, double>(A, alpha, x, beta, y, staged ? device_err_flag() : nullptr,
-                                 (cudaStream_t)stream, staged != 0);
+                                 (cudaStream_t)stream, staged != 0, true);
     });
 }
 
@@ -86,7 +86,7 @@ int jxcpr_bsr_matvec_dev_f32(int nb, int bs, long long nnzb, const int *ia, cons
     return guarded([&] {
         BsrView<float> A{nb, bs, nnzb, ia, ja, a};
         bsr_spmv<float, double>(A, alpha, x, beta, y, staged ? device_err_flag() : nullptr,
-                                (cudaStream_t)stream, staged != 0);
+                                (cudaStream_t)stream, staged != 0, true);
     });
 }
 

@@ -89,10 +89,10 @@ void bsr_decouple_rhs(int nb, int bs, int type, const double *coef, double *rhs,
 // ---- bsr_spmv.cu ---------------------------------------------------------
 // y = alpha*A*x + beta*y with the reference's rounding sequence.  `staged`
 // selects the TMA-staged persistent kernel (requires `err`, a device int set
-// to nonzero if a bounded wait gave up).
+// to nonzero if a bounded wait gave up).  alone: a product by itself, not one of a solve.
 template <typename V, typename X>
 void bsr_spmv(const BsrView<V> &A, X alpha, const X *x, X beta, X *y, int *err, cudaStream_t stream,
-              bool staged = true);
+              bool staged = true, bool alone = false);
 // y = A x for an FP32 x (16-byte aligned, widened before the products: the product with the FP64 vector of
 // the same values), which is also stored as ZT in Z[*i] (device pointers).
 template <typename ZT>
