@@ -11,8 +11,8 @@
 // the start of the pass (the res2 term, and the contributions of rows not yet updated) are formed per entry,
 // so that the chain keeps the products with updated rows only.  Of an 8,000-cell system: a block sweep of 68
 // groups 650 -> 218 us, four sweeps of the level below (150 groups) 8,310 -> 558 us, an application of the
-// preconditioner 15.1 -> 2.6 ms (of an 85,184-cell one 329 -> 35 ms); its setup, which lays the streams out,
-// 10.5 -> 11.9 ms.
+// preconditioner 15.1 -> 2.6 ms (of an 85,184-cell one 340 -> 35, of 264,000 cells 553 -> 82); the setups, which
+// lay the streams out, 6.3 -> 7.8 ms (24.8 -> 32.2, 54 -> 94).
 // The order of operations of every row is the sequential sweep's (jxf_PAMGRelax6,
 // jxfpamg-0220/csrc/operation/relaxations/par_relax_6.c:226-270; jxf_ParBSRHGSRelax,
 // jxfpamg-0220/csrc/amg/par_relax_bsr.c:193-573): results are bit-identical.
