@@ -742,8 +742,9 @@ def roofline_level(G, stream, level, op, value_bytes, vec_bytes, cfg="c1"):
 
 
 def roofline_bsr_spmv(d_ia, d_ja, d_a, s, stream, cfg="c1", staged=0):
-    """The FP64 BSR SpMV y = A x of GMRES on the workload's matrix: bsr_spmv_slab_kernel (the solve's
-    kernel), or with staged = 1 the TMA-staged bsr_spmv_tma_kernel for comparison."""
+    """The FP64 BSR SpMV y = A x on the workload's matrix: bsr_spmv_slab_kernel (3x3 blocks:
+    bsr_spmv_direct_kernel), the solve's kernels, in the form for a product alone; or with staged = 1 the
+    TMA-staged bsr_spmv_tma_kernel for comparison."""
     import torch
 
     from jxpamg_all_b200 import lib
@@ -761,7 +762,8 @@ def roofline_bsr_spmv(d_ia, d_ja, d_a, s, stream, cfg="c1", staged=0):
     sec = _event_time(stream, body, 20)
     bs, nb, nnzb, n = s.block_size, s.num_block_rows, s.nnzb, s.n
     alg = nnzb * (bs * bs * 8 + 4) + (nb + 1) * 4 + 2 * n * 8
-    kname = f"bsr_spmv_tma_kernel<{bs}>" if staged else f"bsr_spmv_{'slab' if bs == 2 else 'direct'}_kernel<{bs}, double>"
+    kname = (f"bsr_spmv_tma_kernel<{bs}>" if staged else "bsr_spmv_slab_kernel<double, NoKeep, true>" if bs == 2
+             else f"bsr_spmv_direct_kernel<{bs}, double>")
     return _roof(f"BSR SpMV y = A x ({kname}, FP64)", alg, sec, cfg, "bsr_spmv_tma/8" if staged else "bsr_spmv/8")
 
 

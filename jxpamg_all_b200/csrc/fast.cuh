@@ -57,7 +57,7 @@ struct LevelMat {
     long long nnz = 0;
     int E = 1;
     int kind = VAL_F64;
-    int sell = 0;
+    int sell = 0;   // 0 CSR, P sliced ELL with P lanes per row
     int chunk = 0;  // sliced ELL in chunk order (stage 2, fk::hgs_chunk): rows per chunk
     int lanes = 1;
     int nstored = 0;

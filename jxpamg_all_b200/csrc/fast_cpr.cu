@@ -234,7 +234,7 @@ void near_columns(LevelMat &M, long long slots, cudaStream_t s) {
 void build_level_mat(int n, int m, long long nnz, int E, const int *ia, const int *ja, const double *a, int kind,
                      int sell, const std::vector<int> &order, const std::vector<int> &seg, const int *order_dev,
                      LevelMat &M, cudaStream_t s) {
-    // sell: 0 CSR, 1 sliced ELL, 2 sliced ELL with two lanes per row (E = 1, FP32 / FP64 values)
+    // sell: 0 CSR, P sliced ELL with P lanes per row (P > 1: E = 1, FP32 / FP64 values)
     if (sell > 1 && (E != 1 || kind == VAL_BF16)) sell = 1;
     M.n = n;
     M.m = m;

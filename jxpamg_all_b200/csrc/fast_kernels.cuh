@@ -685,7 +685,9 @@ __device__ __forceinline__ void block_matvec(const TA M[BS * BS], const TA v[BS]
 }
 
 // The two values of a 2-vector entry j of x (FP32: one 8-byte load; x's base is 8-byte aligned, which
-// the stage-2 launcher checks).
+// the stage-2 launcher checks).  A plain load, as every load of a vector here: the kernel ahead may have been
+// writing x when this one started, which the read-only path does not allow (1.12 M 2x2 rows in FP32: 40.9 us a
+// sweep through it, 41.4 to 42.7 so).
 template <typename TXV, typename TA>
 __device__ __forceinline__ void ld_pair(const TXV *p, int j, TA out[2]) {
     if constexpr (sizeof(TXV) == 4) {
